@@ -19,6 +19,7 @@
 
 #include <cuda_runtime.h>
 
+#include "afx_fp64.cuh"
 #include "afx_launch.hpp"
 
 namespace afx {
@@ -79,14 +80,30 @@ __device__ __forceinline__ void st4(float4* p, const double* v) {
     *p = make_float4((float)v[0], (float)v[1], (float)v[2], (float)v[3]);
 }
 
-__device__ __forceinline__ double dsqrt(double x) { return sqrt(x); }
+__device__ __forceinline__ double dsqrt(double x) { return fp64::root(x); }
 __device__ __forceinline__ float dsqrt(float x) { return sqrtf(x); }
+// quotients: FP64 in integer arithmetic (afx_fp64.cuh), otherwise the type's own;
+// Div holds a denominator that several quotients share
+template <class T> __device__ __forceinline__ T fdiv(const T a, const T b) { return a / b; }
+__device__ __forceinline__ double fdiv(const double a, const double b) { return fp64::div(a, b); }
+template <class T> struct Div {
+    T y;
+    __device__ __forceinline__ explicit Div(const T v) : y(v) {}
+    __device__ __forceinline__ T operator()(const T x) const { return x / y; }
+};
+template <> struct Div<double> {
+    fp64::Den d;
+    __device__ __forceinline__ explicit Div(const double v) : d(fp64::den(v)) {}
+    __device__ __forceinline__ double operator()(const double x) const { return fp64::quot(x, d); }
+};
 __device__ __forceinline__ double dabs(double x) { return fabs(x); }
 __device__ __forceinline__ float dabs(float x) { return fabsf(x); }
 
 // std::min / std::max semantics: min(a,b) = (b < a) ? b : a; max(a,b) = (a < b) ? b : a
 template <class T> __device__ __forceinline__ T smin(T a, T b) { return (b < a) ? b : a; }
 template <class T> __device__ __forceinline__ T smax(T a, T b) { return (a < b) ? b : a; }
+__device__ __forceinline__ double smin(double a, double b) { return fp64::less(b, a) ? b : a; }
+__device__ __forceinline__ double smax(double a, double b) { return fp64::less(a, b) ? b : a; }
 
 // Kernel view of the mesh and physics.
 template <class T>
@@ -166,6 +183,66 @@ __device__ __forceinline__ void roe_flux(const T gamma, const T nx, const T ny, 
                       kF234_1 * (u * (uR - uL) + v * (vR - vL) - V * (VR - VL)) + kF5 * (h + c * V));
 }
 
+// The same in FP64, twice the flux (the caller's face length takes the half,
+// an exact factor): every quotient, root and compare in integer arithmetic
+// with shared denominators, and every factor of two folded into a sum as an
+// exact product or into a denominator's exponent, so each result has the bits
+// of the expression above.  What is left on the FP64 pipe are about 135 sums
+// and products; the compiler's form held it for 18 divisions at 7 and 6
+// roots at 7.6 instructions each beside 180 sums and products.
+__device__ __forceinline__ double entropy_corr64(const double l, const double d, const fp64::Den& d2) {
+    return fp64::less(d, l) ? l : fp64::quot(l * l + d * d, d2);
+}
+__device__ __forceinline__ void roe_flux2(const double gamma, const double nx, const double ny, const double* qL,
+                                          const double* qR, double* f) {
+    using namespace fp64;
+    const Den iL = den(qL[0]), iR = den(qR[0]);
+    const double g1 = gamma - 1.0;
+    const double V_L = quot(qL[1] * nx + qL[2] * ny, iL);
+    const double V_R = quot(qR[1] * nx + qR[2] * ny, iR);
+    const double pL = g1 * (qL[3] - quot(0.5, iL) * (qL[1] * qL[1] + qL[2] * qL[2]));
+    const double pR = g1 * (qR[3] - quot(0.5, iR) * (qR[1] * qR[1] + qR[2] * qR[2]));
+    const double uL = quot(qL[1], iL), uR = quot(qR[1], iR);
+    const double vL = quot(qL[2], iL), vR = quot(qR[2], iR);
+    const double srhoL = root(qL[0]), srhoR = root(qR[0]);
+    const double rho = srhoR * srhoL;
+    const Den is = den(srhoL + srhoR);
+    const double u = quot(uL * srhoL + uR * srhoR, is);
+    const double v = quot(vL * srhoL + vR * srhoR, is);
+    const double h = quot(quot(qL[3] + pL, iL) * srhoL + quot(qR[3] + pR, iR) * srhoR, is);
+    const double q2 = u * u + v * v;
+    const double c = root(g1 * __fma_rn(-0.5, q2, h));
+    const double V = u * nx + v * ny;
+    const double VR = uR * nx + vR * ny;
+    const double VL = uL * nx + vL * ny;
+    const double d = 0.05 * c;
+    const Den d2 = twice(den(d));
+    const double lambda_cm = entropy_corr64(sabs(V - c), d, d2);
+    const double lambda_c = entropy_corr64(sabs(V), d, d2);
+    const double lambda_cp = entropy_corr64(sabs(V + c), d, d2);
+    const Den cc = den(c * c), cc2 = twice(cc);
+    const double dp = pR - pL, dV = VR - VL, rcV = rho * c * dV;
+    const double kF1 = quot(lambda_cm * (dp - rcV), cc2);
+    const double kF234_0 = lambda_c * ((qR[0] - qL[0]) - quot(dp, cc));
+    const double kF234_1 = lambda_c * rho;
+    const double kF5 = quot(lambda_cp * (dp + rcV), cc2);
+    const double cnx = c * nx, cny = c * ny, cV = c * V;
+    f[0] = (V_L * qL[0] + V_R * qR[0]) - (kF1 + kF234_0 + kF5);
+    f[1] = (V_L * qL[1] + pL * nx + V_R * qR[1] + pR * nx) -
+           (kF1 * (u - cnx) + kF234_0 * u + kF234_1 * (uR - uL - dV * nx) + kF5 * (u + cnx));
+    f[2] = (V_L * qL[2] + pL * ny + V_R * qR[2] + pR * ny) -
+           (kF1 * (v - cny) + kF234_0 * v + kF234_1 * (vR - vL - dV * ny) + kF5 * (v + cny));
+    f[3] = (V_L * (qL[3] + pL) + V_R * (qR[3] + pR)) -
+           (__fma_rn(0.5, kF234_0 * q2, kF1 * (h - cV)) + kF234_1 * (u * (uR - uL) + v * (vR - vL) - V * dV) +
+            kF5 * (h + cV));
+}
+__device__ __forceinline__ void roe_flux(const double gamma, const double nx, const double ny, const double* qL,
+                                         const double* qR, double* f) {
+    roe_flux2(gamma, nx, ny, qL, qR, f);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) f[k] *= 0.5;
+}
+
 // Laminar viscous flux at the mean state, physics.h:230-258 with
 // calc_grad_p / calc_grad_temp / calc_grad_u / calc_grad_v (physics.h:33-82).
 template <class T>
@@ -173,27 +250,30 @@ __device__ __forceinline__ void laminar_flux(const T gamma, const T Rgas, const 
                                              const T ny, const T* qL, const T* qR, const T* gx, const T* gy, T* f) {
     T qc[4];
     for (int k = 0; k < 4; ++k) qc[k] = T(0.5) * (qL[k] + qR[k]);
-    const T p = (gamma - T(1)) * (qc[3] - T(0.5) / qc[0] * (qc[1] * qc[1] + qc[2] * qc[2]));
+    const Div<T> i1(qc[0]), i2(qc[0] * qc[0]), i3(T(3));
+    const T p = (gamma - T(1)) * (qc[3] - i1(T(0.5)) * (qc[1] * qc[1] + qc[2] * qc[2]));
     T gp0 = T(2) * gx[3];
-    gp0 -= gx[1] * qc[1] / qc[0] + qc[1] * (gx[1] * qc[0] - gx[0] * qc[1]) / (qc[0] * qc[0]);
-    gp0 -= gx[2] * qc[2] / qc[0] + qc[2] * (gx[2] * qc[0] - gx[0] * qc[2]) / (qc[0] * qc[0]);
+    gp0 -= i1(gx[1] * qc[1]) + i2(qc[1] * (gx[1] * qc[0] - gx[0] * qc[1]));
+    gp0 -= i1(gx[2] * qc[2]) + i2(qc[2] * (gx[2] * qc[0] - gx[0] * qc[2]));
     gp0 *= T(0.5) * (gamma - T(1));
     T gp1 = T(2) * gy[3];
-    gp1 -= gy[1] * qc[1] / qc[0] + qc[1] * (gy[1] * qc[0] - gy[0] * qc[1]) / (qc[0] * qc[0]);
-    gp1 -= gy[2] * qc[2] / qc[0] + qc[2] * (gy[2] * qc[0] - gy[0] * qc[2]) / (qc[0] * qc[0]);
+    gp1 -= i1(gy[1] * qc[1]) + i2(qc[1] * (gy[1] * qc[0] - gy[0] * qc[1]));
+    gp1 -= i1(gy[2] * qc[2]) + i2(qc[2] * (gy[2] * qc[0] - gy[0] * qc[2]));
     gp1 *= T(0.5) * (gamma - T(1));
-    const T gT0 = (T(1) / Rgas) * ((gp0 * qc[0] - gx[0] * p) / (qc[0] * qc[0]));
-    const T gT1 = (T(1) / Rgas) * ((gp1 * qc[0] - gy[0] * p) / (qc[0] * qc[0]));
-    const T gu0 = (qc[0] * gx[1] - qc[1] * gx[0]) / (qc[0] * qc[0]);
-    const T gu1 = (qc[0] * gy[1] - qc[1] * gy[0]) / (qc[0] * qc[0]);
-    const T gv0 = (qc[0] * gx[2] - qc[2] * gx[0]) / (qc[0] * qc[0]);
-    const T gv1 = (qc[0] * gy[2] - qc[2] * gy[0]) / (qc[0] * qc[0]);
-    const T div_v = gu0 + gv1;
-    const T tau_xx = T(2) * mu * (gu0 - div_v / T(3));
-    const T tau_yy = T(2) * mu * (gv1 - div_v / T(3));
+    const T Rinv = fdiv(T(1), Rgas);
+    const T gT0 = Rinv * i2(gp0 * qc[0] - gx[0] * p);
+    const T gT1 = Rinv * i2(gp1 * qc[0] - gy[0] * p);
+    const T gu0 = i2(qc[0] * gx[1] - qc[1] * gx[0]);
+    const T gu1 = i2(qc[0] * gy[1] - qc[1] * gy[0]);
+    const T gv0 = i2(qc[0] * gx[2] - qc[2] * gx[0]);
+    const T gv1 = i2(qc[0] * gy[2] - qc[2] * gy[0]);
+    const T div3 = i3(gu0 + gv1);
+    const T tau_xx = T(2) * mu * (gu0 - div3);
+    const T tau_yy = T(2) * mu * (gv1 - div3);
     const T tau_xy = mu * (gu1 + gv0);
-    const T phi0 = qc[1] / qc[0] * tau_xx + qc[2] / qc[0] * tau_xy + kheat * gT0;
-    const T phi1 = qc[1] / qc[0] * tau_xy + qc[2] / qc[0] * tau_yy + kheat * gT1;
+    const T uc = i1(qc[1]), vc = i1(qc[2]);
+    const T phi0 = uc * tau_xx + vc * tau_xy + kheat * gT0;
+    const T phi1 = uc * tau_xy + vc * tau_yy + kheat * gT1;
     f[1] -= nx * tau_xx + ny * tau_xy;
     f[2] -= nx * tau_xy + ny * tau_yy;
     f[3] -= nx * phi0 + ny * phi1;
@@ -224,38 +304,41 @@ __device__ __forceinline__ void ghost_state(const int type, const T gamma, const
     }
     const T rho = qL[0], rho_u = qL[1], rho_v = qL[2], rho_e = qL[3];
     const T bc_rho = qbc[0], bc_rhou = qbc[1], bc_rhov = qbc[2], bc_rhoe = qbc[3];
-    const T bc_u = bc_rhou / bc_rho;
-    const T bc_v = bc_rhov / bc_rho;
-    const T bc_p = (gamma - T(1)) * (bc_rhoe - T(0.5) / bc_rho * (bc_rhou * bc_rhou + bc_rhov * bc_rhov));
-    const T p = (gamma - T(1)) * (rho_e - T(0.5) / rho * (rho_u * rho_u + rho_v * rho_v));
-    const T c = dsqrt(gamma * p / rho);
-    const T mach = dsqrt(rho_u * rho_u + rho_v * rho_v) / (rho * c);
+    const Div<T> ib(bc_rho), ii(rho), ig(gamma - T(1));
+    const T bc_u = ib(bc_rhou);
+    const T bc_v = ib(bc_rhov);
+    const T bc_p = (gamma - T(1)) * (bc_rhoe - ib(T(0.5)) * (bc_rhou * bc_rhou + bc_rhov * bc_rhov));
+    const T p = (gamma - T(1)) * (rho_e - ii(T(0.5)) * (rho_u * rho_u + rho_v * rho_v));
+    const T c = dsqrt(ii(gamma * p));
+    const Div<T> irc(rho * c);
+    const T mach = irc(dsqrt(rho_u * rho_u + rho_v * rho_v));
     const T inlet_outlet = rho_u * nx + rho_v * ny;
     if (mach > T(1)) {
         if (inlet_outlet < T(0)) {
             qR[0] = bc_rho;
             qR[1] = bc_rho * bc_u;
             qR[2] = bc_rho * bc_v;
-            qR[3] = bc_p / (gamma - T(1)) + T(0.5) * bc_rho * (bc_u * bc_u + bc_v * bc_v);
+            qR[3] = ig(bc_p) + T(0.5) * bc_rho * (bc_u * bc_u + bc_v * bc_v);
         } else {
             qR[0] = rho; qR[1] = rho_u; qR[2] = rho_v; qR[3] = rho_e;
         }
     } else {
         const T pa = bc_p, rhoa = bc_rho, ua = bc_u, va = bc_v;
-        const T pd = p, rhod = rho, ud = rho_u / rho, vd = rho_v / rho;
+        const T pd = p, rhod = rho, ud = ii(rho_u), vd = ii(rho_v);
         const T rho0 = rho, c0 = c;
+        const Div<T> icc(c0 * c0);
         if (inlet_outlet < T(0)) {
             const T pb = T(0.5) * (pa + pd - rho0 * c0 * (nx * (ua - ud) + ny * (va - vd)));
-            qR[0] = rhoa + (pb - pa) / (c0 * c0);
-            qR[1] = qR[0] * (ua - nx * (pa - pb) / (rho0 * c0));
-            qR[2] = qR[0] * (va - ny * (pa - pb) / (rho0 * c0));
-            qR[3] = pb / (gamma - T(1)) + T(0.5) / qR[0] * (qR[1] * qR[1] + qR[2] * qR[2]);
+            qR[0] = rhoa + icc(pb - pa);
+            qR[1] = qR[0] * (ua - irc(nx * (pa - pb)));
+            qR[2] = qR[0] * (va - irc(ny * (pa - pb)));
+            qR[3] = ig(pb) + fdiv(T(0.5), qR[0]) * (qR[1] * qR[1] + qR[2] * qR[2]);
         } else {
             const T pb = pa;
-            qR[0] = rhod + (pb - pd) / (c0 * c0);
-            qR[1] = qR[0] * (ud + nx * (pd - pb) / (rho0 * c0));
-            qR[2] = qR[0] * (va + ny * (pd - pb) / (rho0 * c0));
-            qR[3] = pb / (gamma - T(1)) + T(0.5) / qR[0] * (qR[1] * qR[1] + qR[2] * qR[2]);
+            qR[0] = rhod + icc(pb - pd);
+            qR[1] = qR[0] * (ud + irc(nx * (pd - pb)));
+            qR[2] = qR[0] * (va + irc(ny * (pd - pb)));
+            qR[3] = ig(pb) + fdiv(T(0.5), qR[0]) * (qR[1] * qR[1] + qR[2] * qR[2]);
         }
     }
 }
@@ -274,7 +357,7 @@ __device__ __forceinline__ void face_flux(const KM<T>& m, const int bt, const T 
         roe_flux(m.gamma, nx, ny, qL, qR, f);
         if (VISC == 1) laminar_flux(m.gamma, m.R, m.mu, m.kheat, nx, ny, qL, qR, fgx, fgy, f);
         if (VISC == 2)
-            laminar_flux(m.gamma, m.R, m.mu + mut_f, m.cp * (m.mu / m.PrL + mut_f / m.PrT), nx, ny, qL, qR, fgx, fgy,
+            laminar_flux(m.gamma, m.R, m.mu + mut_f, m.cp * (fdiv(m.mu, m.PrL) + fdiv(mut_f, m.PrT)), nx, ny, qL, qR, fgx, fgy,
                          f);
     } else {
         // VISC 2: the inviscid part of a no-slip wall takes the slip-wall
@@ -291,19 +374,20 @@ __device__ __forceinline__ void face_flux(const KM<T>& m, const int bt, const T 
 template <class T>
 __device__ __forceinline__ void sa_wall_shear(const KM<T>& m, const T nx, const T ny, const T d0x, const T d0y,
                                               const T* q0, T* f) {
-    const T delta = dabs(d0x * nx + d0y * ny);
-    const T u = q0[1] / q0[0], v = q0[2] / q0[0];
+    const Div<T> delta(dabs(d0x * nx + d0y * ny)), i0(q0[0]);
+    const T u = i0(q0[1]), v = i0(q0[2]);
     const T un = u * nx + v * ny;
-    f[1] += m.mu * (u - un * nx) / delta;
-    f[2] += m.mu * (v - un * ny) / delta;
+    f[1] += delta(m.mu * (u - un * nx));
+    f[2] += delta(m.mu * (v - un * ny));
 }
 
 // Spectral radius (c + |V_n|) of one side, solver.h:329-344.
 template <class T>
 __device__ __forceinline__ T face_eig(const T gamma, const T nx, const T ny, const T* q) {
-    const T V = (q[1] * nx + q[2] * ny) / q[0];
-    const T p = (gamma - T(1)) * (q[3] - T(0.5) / q[0] * (q[1] * q[1] + q[2] * q[2]));
-    return dsqrt(p * gamma / q[0]) + dabs(V);
+    const Div<T> i0(q[0]);
+    const T V = i0(q[1] * nx + q[2] * ny);
+    const T p = (gamma - T(1)) * (q[3] - i0(T(0.5)) * (q[1] * q[1] + q[2] * q[2]));
+    return dsqrt(i0(p * gamma)) + dabs(V);
 }
 
 // Venkatakrishnan limiter of one cell-face-variable (solver.h:578-584) and
@@ -312,14 +396,12 @@ template <class T>
 __device__ __forceinline__ T limiter_value(const int kind, const T dqg, const T delta_max, const T delta_min,
                                            const T K3a) {
     if (kind == 0) {
-        if (dqg > T(1e-16)) {
-            return T(1) / dqg * ((delta_max * delta_max + K3a) * dqg + T(2) * dqg * dqg * delta_max) /
-                   (delta_max * delta_max + T(2) * dqg * dqg + delta_max * dqg + K3a);
-        } else if (dqg < T(-1e-16)) {
-            return T(1) / dqg * ((delta_min * delta_min + K3a) * dqg + T(2) * dqg * dqg * delta_min) /
-                   (delta_min * delta_min + T(2) * dqg * dqg + delta_min * dqg + K3a);
-        }
-        return T(1);
+        // the side first: one formula for both signs, so a warp whose lanes
+        // differ in sign forms it once, not twice
+        if (!(dabs(dqg) > T(1e-16))) return T(1);
+        const T dm = dqg > T(0) ? delta_max : delta_min;
+        return T(1) / dqg * ((dm * dm + K3a) * dqg + T(2) * dqg * dqg * dm) /
+               (dm * dm + T(2) * dqg * dqg + dm * dqg + K3a);
     }
     const T dMaxMin2 = (delta_max - delta_min) * (delta_max - delta_min);
     T sig;
@@ -342,6 +424,70 @@ __device__ __forceinline__ T limiter_value(const int kind, const T dqg, const T 
         }
     }
     return sig + (T(1) - sig) * lim;
+}
+
+// The same in FP64 (bits of the expressions above; factors of two as exact
+// products of a fused multiply-add, quotients and compares in integers).
+__device__ __forceinline__ double limiter_value(const int kind, const double dqg, const double delta_max,
+                                                const double delta_min, const double K3a) {
+    using namespace fp64;
+    const uint64_t u = bits_of(dqg), mag = u & 0x7fffffffffffffffull;
+    const bool pos = (u >> 63) == 0;
+    if (kind == 0) {
+        // |dqg| > 1e-16, false for a NaN
+        const bool on = mag > 0x3c9cd2b297d889bcull && mag <= 0x7ff0000000000000ull;
+        const double g = on ? dqg : 1.0;
+        const double dm = pos ? delta_max : delta_min;
+        const double d2 = dm * dm, g2 = g * g;
+        const double num = __fma_rn(2.0, g2 * dm, (d2 + K3a) * g);
+        const double dn = (__fma_rn(2.0, g2, d2) + dm * g) + K3a;
+        const double lim = quot(quot(1.0, den(g)) * num, den(dn));
+        return on ? lim : 1.0;
+    }
+    const double dd = delta_max - delta_min;
+    const double dMaxMin2 = dd * dd;
+    double sig;
+    if (less_equal(dMaxMin2, K3a)) sig = 1.0;
+    else if (less_equal(dMaxMin2, 2.0 * K3a)) {
+        const double y = div(dMaxMin2, K3a) - 1.0;
+        sig = 2.0 * y * y * y - 3.0 * y * y + 1.0;
+    } else sig = 0.0;
+    double lim = 1.0;
+    if (less(sig, 1.0)) {
+        // |dqg| > 1e-14, false for a NaN
+        const bool on = mag > 0x3d06849b86a12b9bull && mag <= 0x7ff0000000000000ull;
+        const double y = on ? div(pos ? delta_max : delta_min, dqg) : 2.0;
+        const double YT = 2.0;
+        const double a = 1.0 / (YT * YT) - 2.0 / (YT * YT * YT);
+        const double b = -3.0 / 2.0 * a * YT - 0.5 / YT;
+        lim = less_equal(YT, y) ? 1.0 : a * y * y * y + b * y * y + y;
+    }
+    return sig + (1.0 - sig) * lim;
+}
+
+// F times the face length.  FP64 without a viscous term: twice the flux times
+// half the length, an exact factor.
+template <class T, int VISC>
+__device__ __forceinline__ void face_flux_length(const KM<T>& m, const int bt, const T nx, const T ny, const T* qL,
+                                                 const T* qR, const T* fgx, const T* fgy, const T L, T* fl,
+                                                 const T mut_f) {
+    face_flux<T, VISC>(m, bt, nx, ny, qL, qR, fgx, fgy, fl, mut_f);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) fl[k] = fl[k] * L;
+}
+template <>
+__device__ __forceinline__ void face_flux_length<double, 0>(const KM<double>& m, const int bt, const double nx,
+                                                            const double ny, const double* qL, const double* qR,
+                                                            const double*, const double*, const double L, double* fl,
+                                                            const double) {
+    double qb[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) qb[k] = qR[k];
+    if (!two_sided(bt)) ghost_state(bt, m.gamma, nx, ny, qL, qR, qb);
+    roe_flux2(m.gamma, nx, ny, qL, qb, fl);
+    const double h = 0.5 * L;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) fl[k] = fl[k] * h;
 }
 
 }  // namespace dev

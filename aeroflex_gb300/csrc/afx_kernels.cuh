@@ -87,12 +87,20 @@ __global__ void __launch_bounds__(256) k_prep(const KM<T> m, const V4<S>* __rest
                 eigsum += eig * Lg.x;
             }
             if (GRAD && !m.lsq) {
-                T qRv[4];
-                ghost_state(bt, m.gamma, n.x, n.y, q0c, q1c, qRv);
+                // an interior face's far value is the mean of both states: its
+                // half goes with the weight (an exact factor)
                 const T g = Lg.y;
+                T qRv[4], gr = g;
+                if (bt == BT_INTERNAL) {
+                    gr = T(0.5) * g;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) qRv[k] = q0c[k] + q1c[k];
+                } else {
+                    ghost_state(bt, m.gamma, n.x, n.y, q0c, q1c, qRv);
+                }
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    const T fk = (q0c[k] * (T(1) - g) + qRv[k] * g) * Lg.x;
+                    const T fk = (q0c[k] * (T(1) - g) + qRv[k] * gr) * Lg.x;
                     if (own0) {
                         sgx[k] += fk * n.x;
                         sgy[k] += fk * n.y;
@@ -117,7 +125,7 @@ __global__ void __launch_bounds__(256) k_prep(const KM<T> m, const V4<S>* __rest
         }
     }
     const T A = __ldg(&m.area[i]);
-    if (DTP) dt[i] = m.cfl * A / eigsum;
+    if (DTP) dt[i] = fdiv(m.cfl * A, eigsum);
     if (!GRAD) return;
     T gxi[4], gyi[4];
     if (m.lsq) {
@@ -152,10 +160,11 @@ __global__ void __launch_bounds__(256) k_prep(const KM<T> m, const V4<S>* __rest
             }
         }
     } else {
+        const Div<T> iA(A);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            gxi[k] = sgx[k] / A;
-            gyi[k] = sgy[k] / A;
+            gxi[k] = iA(sgx[k]);
+            gyi[k] = iA(sgy[k]);
         }
     }
     V4<T> vx, vy;
@@ -267,10 +276,11 @@ __device__ __forceinline__ void reconstruct(const T* q, const T* gxc, const T* g
 template <class T>
 __device__ __forceinline__ void face_gradient(const T* qa, const T* qb, const T* gxa, const T* gya, const T* gxb,
                                               const T* gyb, const V4<T> t, T* fgx, T* fgy) {
-    const T t0 = t.x, t1 = t.y, lij = t.z;
+    const T t0 = t.x, t1 = t.y;
+    const Div<T> ilij(t.z);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const T grad_dir = (qa[k] - qb[k]) / lij;
+        const T grad_dir = ilij(qa[k] - qb[k]);
         const T gxb_ = (gxa[k] + gxb[k]) * T(0.5);
         const T gyb_ = (gya[k] + gyb[k]) * T(0.5);
         const T grad_dot = gxb_ * t0 + gyb_ * t1;
@@ -386,8 +396,9 @@ __device__ __forceinline__ void stage_epilogue(const StageOut<T, S>& o, const in
     double sq = extra_sq;
     if (active) {
         T R[4];
+        const Div<T> iA(A);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) R[k] = Rsum[k] / A;
+        for (int k = 0; k < 4; ++k) R[k] = iA(Rsum[k]);
         if (o.case_done && o.mode < 2 && __ldg(&o.case_done[__ldg(&o.case_of[i])])) {
             // a case that has stopped keeps its state
             if (o.mode == 0) {
@@ -434,9 +445,10 @@ __device__ __forceinline__ void stage_epilogue(const StageOut<T, S>& o, const in
             double q0[4];
             ld4(&o.q0[i], q0);
             const double dtd = (double)dti;
+            const double ar = o.alpha * o.relax;  // alpha is a power of two: an exact product
             double qn[4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) qn[k] = q0[k] + (double)R[k] * dtd * o.alpha * o.relax;
+            for (int k = 0; k < 4; ++k) qn[k] = q0[k] + (double)R[k] * dtd * ar;
             if (o.mode == 0) {
                 V4<S> v;
                 st4(&v, qn);
@@ -655,16 +667,20 @@ __device__ __forceinline__ void face_flux_at(const KM<T>& m, const int f, const 
         else ld4c<T>(&m.bq[-cc.y - 1], qb);
         face_gradient(qa, qb, gx0, gy0, gx1, gy1, ldv4<T>(&m.ft[f]), fgx, fgy);
     }
-    T F[4];
     T mut_f = T(0);
     if (VISC == 2 && two_sided(bt)) mut_f = T(0.5) * (__ldg(&m.mut[cc.x]) + __ldg(&m.mut[cc.y]));
-    face_flux<T, VISC>(m, bt, n.x, n.y, qL, qR, fgx, fgy, F, mut_f);
-    if (VISC == 2 && bt == BT_WALL) {
-        const V2<T> d0 = __ldg(&m.fd0[f]);
-        sa_wall_shear(m, n.x, n.y, d0.x, d0.y, q0, F);
-    }
+    if (VISC == 2) {
+        T F[4];
+        face_flux<T, VISC>(m, bt, n.x, n.y, qL, qR, fgx, fgy, F, mut_f);
+        if (bt == BT_WALL) {
+            const V2<T> d0 = __ldg(&m.fd0[f]);
+            sa_wall_shear(m, n.x, n.y, d0.x, d0.y, q0, F);
+        }
 #pragma unroll
-    for (int k = 0; k < 4; ++k) fl[k] = F[k] * L;
+        for (int k = 0; k < 4; ++k) fl[k] = F[k] * L;
+    } else {
+        face_flux_length<T, VISC>(m, bt, n.x, n.y, qL, qR, fgx, fgy, L, fl, mut_f);
+    }
     *btp = cc.y >= 0 ? -1 : bt;  // -1: interior face
 }
 
@@ -755,7 +771,7 @@ __global__ void __launch_bounds__(256, 8) k_resid_tile(const KM<T> m, const Tile
         }
         A = __ldg(&m.area[i]);
         if (EIG) {
-            dti = m.cfl * A / eigsum;
+            dti = fdiv(m.cfl * A, eigsum);
             o.dt[i] = dti;
         } else if (o.mode < 2) {
             dti = o.dt[i];
@@ -807,7 +823,7 @@ __global__ void __launch_bounds__(256) k_cell_sum(const KM<T> m, const V4<T>* __
         }
         A = __ldg(&m.area[i]);
         if (DT) {
-            dti = m.cfl * A / eigsum;
+            dti = fdiv(m.cfl * A, eigsum);
             o.dt[i] = dti;
         } else if (o.mode < 2) {
             dti = o.dt[i];
