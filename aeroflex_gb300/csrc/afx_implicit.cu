@@ -74,41 +74,31 @@ __device__ __forceinline__ void ldt(const float4* p, float* v) {
 __device__ __forceinline__ void stt(d4* p, const double* v) { st4(p, v); }
 __device__ __forceinline__ void stt(float4* p, const float* v) { *p = make_float4(v[0], v[1], v[2], v[3]); }
 
-// y += sgn * B x for a 4x4 block (row-major) in T.  Blocks start on a
-// 16-byte boundary (16 T per block, buffers from cudaMalloc), so each row is
-// read with 16-byte vector loads: a cell's block is then 4 (FP32) or 8 (FP64)
-// load instructions, not 16 scattered scalar ones.
+// Row r of a 4x4 block (row-major) times x: the row is one (FP32) or two
+// (FP64) 16-byte chunks, `stride` chunks apart.
 template <class T>
-__device__ __forceinline__ void bmv_add(const T* __restrict__ B, const T* x, T* y, const T sgn);
+__device__ __forceinline__ T row_dot(const T* __restrict__ chunk, const size_t stride, const T* x);
 template <>
-__device__ __forceinline__ void bmv_add<float>(const float* __restrict__ B, const float* x, float* y,
-                                               const float sgn) {
-    const float4* b = reinterpret_cast<const float4*>(B);
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const float4 row = __ldg(&b[r]);
-        float s = 0;
-        s += row.x * x[0];
-        s += row.y * x[1];
-        s += row.z * x[2];
-        s += row.w * x[3];
-        y[r] += sgn * s;
-    }
+__device__ __forceinline__ float row_dot<float>(const float* __restrict__ chunk, const size_t, const float* x) {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(chunk));
+    float t = 0;
+    t += a.x * x[0];
+    t += a.y * x[1];
+    t += a.z * x[2];
+    t += a.w * x[3];
+    return t;
 }
 template <>
-__device__ __forceinline__ void bmv_add<double>(const double* __restrict__ B, const double* x, double* y,
-                                                const double sgn) {
-    const double2* b = reinterpret_cast<const double2*>(B);
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const double2 u = __ldg(&b[2 * r]), v = __ldg(&b[2 * r + 1]);
-        double s = 0;
-        s += u.x * x[0];
-        s += u.y * x[1];
-        s += v.x * x[2];
-        s += v.y * x[3];
-        y[r] += sgn * s;
-    }
+__device__ __forceinline__ double row_dot<double>(const double* __restrict__ chunk, const size_t stride,
+                                                  const double* x) {
+    const double2* c = reinterpret_cast<const double2*>(chunk);
+    const double2 u = __ldg(c), v = __ldg(c + stride);
+    double t = 0;
+    t += u.x * x[0];
+    t += u.y * x[1];
+    t += v.x * x[2];
+    t += v.y * x[3];
+    return t;
 }
 
 // Batch: a cell of a case that has stopped takes no part in the linear
@@ -231,40 +221,12 @@ __device__ __forceinline__ size_t ell_at(const int N, const int p, const int s, 
     constexpr int W = Ell16<T>::W, CPB = Ell16<T>::CPB;
     return ((size_t)(s * CPB + k / W) * N + p) * W + (k % W);
 }
-// y += sgn * O x for the block of slot s of row p
+// row r of the block of slot s of row p, times x
 template <class T>
-__device__ __forceinline__ void ell_mv_add(const T* __restrict__ off, const int N, const int p, const int s,
-                                           const T* x, T* y, const T sgn);
-template <>
-__device__ __forceinline__ void ell_mv_add<float>(const float* __restrict__ off, const int N, const int p,
-                                                  const int s, const float* x, float* y, const float sgn) {
-    const float4* b = reinterpret_cast<const float4*>(off);
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const float4 row = __ldg(&b[(size_t)(s * 4 + r) * N + p]);
-        float t = 0;
-        t += row.x * x[0];
-        t += row.y * x[1];
-        t += row.z * x[2];
-        t += row.w * x[3];
-        y[r] += sgn * t;
-    }
-}
-template <>
-__device__ __forceinline__ void ell_mv_add<double>(const double* __restrict__ off, const int N, const int p,
-                                                   const int s, const double* x, double* y, const double sgn) {
-    const double2* b = reinterpret_cast<const double2*>(off);
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const double2 u = __ldg(&b[(size_t)(s * 8 + 2 * r) * N + p]);
-        const double2 v = __ldg(&b[(size_t)(s * 8 + 2 * r + 1) * N + p]);
-        double t = 0;
-        t += u.x * x[0];
-        t += u.y * x[1];
-        t += v.x * x[2];
-        t += v.y * x[3];
-        y[r] += sgn * t;
-    }
+__device__ __forceinline__ T ell_row(const T* __restrict__ off, const int N, const int p, const int s, const int r,
+                                     const T* x) {
+    constexpr int W = Ell16<T>::W, CPB = Ell16<T>::CPB;
+    return row_dot<T>(off + ((size_t)(s * CPB + r * (CPB / 4)) * N + p) * W, (size_t)N, x);
 }
 
 // Diagonal block A/dt I + sum (own: J, other: -K) of row p and its inverse
@@ -477,34 +439,78 @@ __global__ void __launch_bounds__(128) k_imp_ilu(const Ell e, const int N, const
 }
 
 // --------------------------------------------------------- linear algebra
-// y = M x over the rows (diagonal block, then the slots in face order)
-template <class T>
-__global__ void __launch_bounds__(256) k_imp_spmv(const int n_rows, const Ell e, const T* __restrict__ dblk,
-                                                  const T* __restrict__ off,
-                                                  const typename B4<T>::type* __restrict__ x,
-                                                  typename B4<T>::type* __restrict__ y, const int* __restrict__ stop,
-                                                  const int* __restrict__ case_done) {
-    if (stop && *stop) return;
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n_rows) return;
-    if (held(e.case_row, case_done, p)) {
-        const T z[4] = {0, 0, 0, 0};
-        stt(&y[p], z);
-        return;
-    }
-    T xi[4], yi[4] = {0, 0, 0, 0};
-    ldt(&x[p], xi);
-    bmv_add<T>(dblk + 16 * (size_t)p, xi, yi, T(1));
+// RT threads per row, each with NC = 4 / RT rows of its 4x4 blocks.  One
+// thread per row (16-byte chunks side by side in a warp's loads) streams best
+// when there are rows enough to fill the GPU; a colour of a mesh of tens of
+// thousands of cells has only a few thousand, and then four threads per row
+// put four times as many warps to work (in FP64 a thread's 80 fused
+// multiply-adds alone hold the two FP64 lanes of its SM for microseconds).
+// The sums run in the order of the block form either way, so the results do
+// not depend on RT.  Bound by latency at these sizes: a colour of 3,300 rows in
+// FP64 took 8.0 us with one thread per row in blocks of 256, 3.8 us with four.
+template <class T, int RT>
+__device__ __forceinline__ void row_load(const T* __restrict__ r, const size_t p, const int c, T* s) {
+    if constexpr (RT == 1) ldt(reinterpret_cast<const typename B4<T>::type*>(r) + p, s);
+    else s[0] = r[4 * p + c];
+}
+template <class T, int RT>
+__device__ __forceinline__ void row_store(T* r, const size_t p, const int c, const T* s) {
+    if constexpr (RT == 1) stt(reinterpret_cast<typename B4<T>::type*>(r) + p, s);
+    else r[4 * p + c] = s[0];
+}
+
+// rows of M x for row p
+template <class T, int RT>
+__device__ __forceinline__ void spmv_row(const int n_rows, const Ell& e, const T* __restrict__ dblk,
+                                         const T* __restrict__ off, const T* __restrict__ x, const int p, const int c,
+                                         T* y) {
+    constexpr int NC = 4 / RT;
+    const typename B4<T>::type* x4 = reinterpret_cast<const typename B4<T>::type*>(x);
+    T xi[4];
+    ldt(&x4[p], xi);
     const int4 col = __ldg(&e.col[p]);
+#pragma unroll
+    for (int r = 0; r < NC; ++r) y[r] = row_dot<T>(dblk + 16 * (size_t)p + 4 * (c + r), 1, xi);
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
         const int q = pick(col, s);
         if (q < 0) continue;
         T xo[4];
-        ldt(&x[q], xo);
-        ell_mv_add<T>(off, n_rows, p, s, xo, yi, T(1));
+        ldt(&x4[q], xo);
+#pragma unroll
+        for (int r = 0; r < NC; ++r) y[r] += ell_row<T>(off, n_rows, p, s, c + r, xo);
     }
-    stt(&y[p], yi);
+}
+
+// y = M x over the rows (diagonal block, then the slots in face order)
+template <class T>
+__global__ void __launch_bounds__(256) k_imp_spmv(const int n_rows, const Ell e, const T* __restrict__ dblk,
+                                                  const T* __restrict__ off, const T* __restrict__ x,
+                                                  T* __restrict__ y, const int* __restrict__ stop,
+                                                  const int* __restrict__ case_done) {
+    if (stop && *stop) return;
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n_rows) return;
+    T yr[4] = {0, 0, 0, 0};
+    if (!held(e.case_row, case_done, p)) spmv_row<T, 1>(n_rows, e, dblk, off, x, p, 0, yr);
+    row_store<T, 1>(y, p, 0, yr);
+}
+
+// Rows of D_p^-1 s; with RT = 4 the row's four threads hold one component of s each
+template <class T, int RT>
+__device__ __forceinline__ void dinv_row(const T* __restrict__ dinv, const int p, const int c, const T* s, T* x) {
+    constexpr int NC = 4 / RT;
+    T sv[4];
+    if constexpr (RT == 1) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) sv[k] = s[k];
+    } else {
+        const unsigned lanes = 0xfu << (threadIdx.x & 28);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) sv[k] = __shfl_sync(lanes, s[0], k, RT);
+    }
+#pragma unroll
+    for (int r = 0; r < NC; ++r) x[r] = row_dot<T>(dinv + 16 * (size_t)p + 4 * (c + r), 1, sv);
 }
 
 // One colour (rows c0 .. c0+n-1) of a block Gauss-Seidel sweep:
@@ -512,48 +518,86 @@ __global__ void __launch_bounds__(256) k_imp_spmv(const int n_rows, const Ell e,
 // given (the current Krylov vector).  In the forward sweep only rows of
 // lower colours (q < c0) are read: the higher colours have no value yet
 // (zero start).
-template <class T>
-__global__ void __launch_bounds__(256) k_imp_gs(const Ell e, const int N, const T* __restrict__ dinv,
-                                                const T* __restrict__ off, const int c0, const int n, const T* __restrict__ rbase,
-                                                const int* __restrict__ rk, const long long stride,
-                                                typename B4<T>::type* __restrict__ x, const int* __restrict__ stop,
+template <class T, int RT>
+__global__ void __launch_bounds__(128) k_imp_gs(const Ell e, const int N, const T* __restrict__ dinv,
+                                                const T* __restrict__ off, const int c0, const int n,
+                                                const T* __restrict__ rbase, const int* __restrict__ rk,
+                                                const long long stride, T* x, const int* __restrict__ stop,
                                                 const int* __restrict__ case_done, const bool fwd) {
+    constexpr int NC = 4 / RT;
     if (stop && *stop) return;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    const typename B4<T>::type* r =
-        reinterpret_cast<const typename B4<T>::type*>(rbase + (rk ? (long long)*rk * stride : 0));
-    const int p = c0 + t;
+    if (t >= n * RT) return;
+    const T* r = rbase + (rk ? (long long)*rk * stride : 0);
+    const int p = c0 + t / RT, c = NC * (t % RT);
+    T xr[NC];
     if (held(e.case_row, case_done, p)) {
-        const T z[4] = {0, 0, 0, 0};
-        stt(&x[p], z);
+#pragma unroll
+        for (int k = 0; k < NC; ++k) xr[k] = T(0);
+        row_store<T, RT>(x, p, c, xr);
         return;
     }
-    T s[4];
-    ldt(&r[p], s);
+    T s[NC];
+    row_load<T, RT>(r, p, c, s);
     const int4 col = __ldg(&e.col[p]);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const int q = pick(col, k);
         if (q < 0 || (fwd && q >= c0)) continue;
         T xo[4];
-        ldt(&x[q], xo);
-        ell_mv_add<T>(off, N, p, k, xo, s, T(-1));
+        ldt(reinterpret_cast<const typename B4<T>::type*>(x) + q, xo);
+#pragma unroll
+        for (int j = 0; j < NC; ++j) s[j] -= ell_row<T>(off, N, p, k, c + j, xo);
     }
-    T xi[4] = {0, 0, 0, 0};
-    bmv_add<T>(dinv + 16 * (size_t)p, s, xi, T(1));
-    stt(&x[p], xi);
+    dinv_row<T, RT>(dinv, p, c, s, xr);
+    row_store<T, RT>(x, p, c, xr);
+}
+
+// The start of an Arnoldi step: v_k = w * scale[0] over all rows, and the
+// first colour of the forward sweep, x_p = D_p^-1 v_p, over its n0 rows.
+template <class T, int RT>
+__global__ void __launch_bounds__(128) k_imp_scale_gs(const Ell e, const int n_rows, const T* __restrict__ dinv,
+                                                      const int n0, const T* __restrict__ w,
+                                                      const double* __restrict__ scale, T* __restrict__ vbase,
+                                                      const int* __restrict__ vk, T* __restrict__ x,
+                                                      const int* __restrict__ stop, const int* __restrict__ case_done) {
+    constexpr int NC = 4 / RT;
+    if (*stop) return;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, p = t / RT, c = NC * (t % RT);
+    if (p >= n_rows) return;
+    const T sc = (T)scale[0];
+    T s[NC], xr[NC];
+    row_load<T, RT>(w, p, c, s);
+#pragma unroll
+    for (int k = 0; k < NC; ++k) s[k] *= sc;
+    row_store<T, RT>(vbase + (long long)*vk * (4 * (long long)n_rows), p, c, s);
+    if (p >= n0) return;
+    dinv_row<T, RT>(dinv, p, c, s, xr);
+    if (held(e.case_row, case_done, p)) {
+#pragma unroll
+        for (int k = 0; k < NC; ++k) xr[k] = T(0);
+    }
+    row_store<T, RT>(x, p, c, xr);
 }
 
 // Dot products against the Krylov basis v_0..v_{nv-1} (v_j = V + j*n) in
 // one pass, with the Gram-Schmidt update fused in:
-//   MODE 0: out_j = v_j . w
 //   MODE 1: w -= sum_j hin_j v_j, then out_j = v_j . w   (CGS pass 1 + dots of pass 2)
-//   MODE 2: w -= sum_j hin_j v_j, then out_0 = w . w     (CGS pass 2 + the norm)
-// Each block writes its partial sums; the last block to finish adds them in
-// a fixed pattern (DOT_G threads per output, each over a fixed stride of
-// blocks, then a fixed shuffle tree), so the result is deterministic, and
-// re-arms the counter.
+//   MODE 2: w -= sum_j hin_j v_j, then out_0 = w . w     (CGS pass 2 + the norm; nv = 0: the norm alone)
+// (the dots of pass 1 are formed with w = M x, k_imp_spmv_dots)
+// The per-thread sums of all outputs are reduced across a warp together: a
+// butterfly that halves the outputs a lane holds at every step takes 31 (16
+// for up to 16 outputs) additions of a warp instead of 5 per output -- in
+// FP64 each of them holds the FP64 pipe for 18.6 cycles, and this reduction
+// was most of the kernel.  FP32 sums are added as unevaluated pairs (error-free
+// two-sum, 48 bits) on the FP32 lanes; double takes over after it.  Each block
+// writes its partial sums; the last block to finish adds them in a fixed
+// pattern (a warp per group of blocks, then over the warps), so the result is
+// deterministic, and re-arms the counter.  In MODE 2 of an Arnoldi step one more block applies the earlier
+// Givens rotations to the new column meanwhile, and the last block adds the
+// new rotation.  One Arnoldi step's product, three passes, column and scaling
+// at 16k rows in FP64: 91 -> 42 us in 4 launches instead of 6; at 131k rows in
+// FP32: 68 -> 41 us.
 // 16-byte chunks of a vector in T, their dot product and w -= h v
 template <class T> struct Vec16;
 template <> struct Vec16<float> { using type = float4; static constexpr int W = 4; };
@@ -568,198 +612,339 @@ __device__ __forceinline__ void vsub(float4& w, const float h, const float4 v) {
 __device__ __forceinline__ void vsub(double2& w, const double h, const double2 v) {
     w.x -= h * v.x; w.y -= h * v.y;
 }
-__device__ __forceinline__ void vscale(float4& a, const float s) { a.x *= s; a.y *= s; a.z *= s; a.w *= s; }
-__device__ __forceinline__ void vscale(double2& a, const double s) { a.x *= s; a.y *= s; }
 
-constexpr int DOT_G = 8;  // threads of the last block per output
-static_assert(DOT_THREADS / DOT_G >= GM_M + 1, "one group per output");
-
-template <class T, int MODE>
-__global__ void __launch_bounds__(DOT_THREADS, MODE == 1 ? 1 : 2) k_imp_dots(const int n, int nv, const int* __restrict__ nvk,
-                                                          const T* __restrict__ V, T* __restrict__ w,
-                                                          const double* __restrict__ hin, double* __restrict__ part,
-                                                          unsigned* __restrict__ counter, double* __restrict__ out,
-                                                          const int* __restrict__ stop) {
-    __shared__ double sh[DOT_THREADS / 32][GM_M + 1];
-    __shared__ T hs[GM_M + 1];
-    __shared__ bool last;
-    if (stop && *stop) return;
-    if (nvk) nv = *nvk + 1;  // v_0 .. v_k of the current Arnoldi step
-    const int nout = MODE == 2 ? 1 : nv;
-    if (MODE > 0) {
-        if ((int)threadIdx.x < nv) hs[threadIdx.x] = (T)hin[threadIdx.x];
-        __syncthreads();
+// A partial sum on its way through the warp's reduction
+template <class T> struct Part;
+template <> struct Part<double> {
+    double v;
+    __device__ __forceinline__ void set(const double a) { v = a; }
+    __device__ __forceinline__ double get() const { return v; }
+    __device__ __forceinline__ Part from(const int m) const {
+        Part o;
+        o.v = __shfl_xor_sync(0xffffffffu, v, m);
+        return o;
     }
-    // per-thread partial sums in T over 16-byte chunks of the vectors (a few
-    // chunks each; n is 4 * cells, so whole chunks), then double
-    using VT = typename Vec16<T>::type;
-    const int nc = n / Vec16<T>::W;
-    const VT* __restrict__ Vv = reinterpret_cast<const VT*>(V);
-    VT* __restrict__ wv = reinterpret_cast<VT*>(w);
-    T acc[GM_M + 1];
+    __device__ __forceinline__ void add(const Part& o) { v += o.v; }
+};
+template <> struct Part<float> {
+    float h, l;  // unevaluated sum
+    __device__ __forceinline__ void set(const float a) { h = a; l = 0.f; }
+    __device__ __forceinline__ double get() const { return (double)h + (double)l; }
+    __device__ __forceinline__ Part from(const int m) const {
+        Part o;
+        o.h = __shfl_xor_sync(0xffffffffu, h, m);
+        o.l = __shfl_xor_sync(0xffffffffu, l, m);
+        return o;
+    }
+    __device__ __forceinline__ void add(const Part& o) {  // Knuth's two-sum of the leading parts
+        const float s = __fadd_rn(h, o.h), b = __fadd_rn(s, -h);
+        const float err = __fadd_rn(__fadd_rn(h, -__fadd_rn(s, -b)), __fadd_rn(o.h, -b));
+        l = __fadd_rn(__fadd_rn(l, o.l), err);
+        h = s;
+    }
+};
+// Sums of acc[0..W-1] over the warp; lane j (mod W) gets output j
+template <int W, class T>
+__device__ __forceinline__ Part<T> warp_sums(const T* acc, const int lane) {
+    Part<T> a[W];
 #pragma unroll
-    for (int j = 0; j <= GM_M; ++j) acc[j] = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nc; i += gridDim.x * blockDim.x) {
-        VT wi = wv[i];
-        if (MODE == 0) {
+    for (int j = 0; j < W; ++j) a[j].set(acc[j]);
 #pragma unroll
-            for (int j = 0; j <= GM_M; ++j)
-                if (j < nv) acc[j] += vdot(Vv[(size_t)j * nc + i], wi);
-        } else {
-            // MODE 1 keeps the basis chunks in registers for the second
-            // product (one block per SM; the loads of a chunk are all in
-            // flight at once)
-            VT vv[GM_M + 1];
+    for (int m = W / 2; m > 0; m >>= 1) {
+        const bool up = lane & m;
 #pragma unroll
-            for (int j = 0; j <= GM_M; ++j)
-                if (j < nv) {
-                    vv[j] = Vv[(size_t)j * nc + i];
-                    vsub(wi, hs[j], vv[j]);
-                }
-            wv[i] = wi;
-            if (MODE == 1) {
-#pragma unroll
-                for (int j = 0; j <= GM_M; ++j)
-                    if (j < nv) acc[j] += vdot(vv[j], wi);
-            } else {
-                acc[0] += vdot(wi, wi);
-            }
+        for (int j = 0; j < m; ++j) {
+            const Part<T> give = up ? a[j] : a[j + m];
+            a[j] = up ? a[j + m] : a[j];
+            a[j].add(give.from(m));
         }
     }
+#pragma unroll
+    for (int m = W; m < 32; m <<= 1) a[0].add(a[0].from(m));
+    return a[0];
+}
+
+// Arnoldi step j = c->k, classical Gram-Schmidt twice: h1 (first pass) and
+// h2 (second pass) sum to column j.  givens_column applies the rotations of
+// the earlier steps to it (one warp, staged in shared memory so the chain runs
+// on shared memory, not on dependent global loads) while the second pass's
+// update is still running; givens_finish adds the subdiagonal entry sqrt(ww),
+// its rotation and the residual estimate.
+struct GivensCol {
+    double col[GM_M + 1], cs[GM_M], sn[GM_M];
+};
+__device__ __forceinline__ void givens_column(GmresCtl* c, const double* __restrict__ h1,
+                                              const double* __restrict__ h2, GivensCol& g) {
+    const int lane = threadIdx.x, j = c->k;
+    for (int t = lane; t <= j; t += 32) g.col[t] = h1[t] + h2[t];
+    for (int t = lane; t < j; t += 32) {
+        g.cs[t] = c->cs[t];
+        g.sn[t] = c->sn[t];
+    }
+    __syncwarp();
+    if (lane == 0) {
+        double a = g.col[0];
+        for (int i = 0; i < j; ++i) {
+            const double b = g.col[i + 1];
+            g.col[i] = g.cs[i] * a + g.sn[i] * b;
+            a = -g.sn[i] * a + g.cs[i] * b;
+        }
+        g.col[j] = a;
+    }
+    __syncwarp();
+    for (int t = lane; t <= j; t += 32) c->H[t + (GM_M + 1) * j] = g.col[t];
+}
+__device__ __forceinline__ void givens_finish(GmresCtl* c, const double ww, double* __restrict__ scale) {
+    const int j = c->k;
+    double* col = c->H + (GM_M + 1) * j;
+    const double hn = sqrt(fmax(ww, 0.0));
+    c->hnext = hn;
+    scale[0] = hn > 0 ? 1.0 / hn : 0.0;
+    const double a = __ldcg(&col[j]), b = hn;
+    const double r = sqrt(a * a + b * b);
+    const double cj = r > 0 ? a / r : 1.0, sj = r > 0 ? b / r : 0.0;
+    c->cs[j] = cj;
+    c->sn[j] = sj;
+    col[j] = r;
+    col[j + 1] = 0;
+    const double g = c->g[j];
+    const double res = fabs(sj * g);
+    const int iters = c->iters + 1;
+    c->g[j + 1] = -sj * g;
+    c->g[j] = cj * g;
+    c->res = res;
+    c->k = j + 1;
+    c->iters = iters;
+    const int st = (res <= c->tol || j + 1 == GM_M || hn == 0 || iters >= c->max_iters) ? 1 : 0;
+    c->stop = st;
+    if (c->graph) cudaGraphSetConditional(c->hin, st ? 0 : 1);
+}
+
+// Basis vectors are read DOT_U at a time, all loads of a group before its
+// arithmetic: one after the other each load would wait out its own latency
+// (3 TB/s at 32 MB of basis).
+constexpr int DOT_U = 8;
+static_assert((GM_M + 2) % DOT_U == 0, "whole groups");
+
+// The block's and, in the last block to finish, the whole sum of the threads'
+// acc[0..nout-1] over blocks 0..nblk-1 of NT threads; true in the last block's
+// first nout threads, with the sums in `total`.  A block with blk < 0 only
+// counts itself.
+template <class T, int NT, bool ONE>
+__device__ __forceinline__ bool grid_sums(const T* acc, const int nout, const int blk, const int nblk,
+                                          double* __restrict__ part, unsigned* __restrict__ counter, double& total) {
+    const bool adds = blk >= 0;
+    constexpr int NW = NT / 32;
+    __shared__ double sh[NW][32];
+    __shared__ bool last;
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-#pragma unroll
-    for (int j = 0; j <= GM_M; ++j) {
-        if (j >= nout) break;
-        double v = (double)acc[j];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if (lane == 0) sh[wp][j] = v;
+    if (adds) {
+        if (ONE) {
+            const Part<T> v = warp_sums<1, T>(acc, lane);
+            if (lane == 0) sh[wp][0] = v.get();
+        } else if (nout > 16) {
+            const Part<T> v = warp_sums<32, T>(acc, lane);
+            if (lane < nout) sh[wp][lane] = v.get();
+        } else {
+            const Part<T> v = warp_sums<16, T>(acc, lane);
+            if (lane < nout) sh[wp][lane] = v.get();
+        }
     }
     __syncthreads();
-    if ((int)threadIdx.x < nout) {
+    if (adds && (int)threadIdx.x < nout) {
         double t = 0;
-        for (int k = 0; k < (int)(blockDim.x >> 5); ++k) t += sh[k][threadIdx.x];
-        part[(size_t)blockIdx.x * nout + threadIdx.x] = t;
+#pragma unroll
+        for (int k = 0; k < NW; ++k) t += sh[k][threadIdx.x];
+        part[(size_t)blk * nout + threadIdx.x] = t;
         __threadfence();  // the partials are visible before the block is counted
     }
     __syncthreads();
     if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
     __syncthreads();
-    if (!last) return;
+    if (!last) return false;
     __threadfence();
-    // the last block: DOT_G threads per output, each over blocks g, g+DOT_G,
-    // ... (L2 reads, several in flight), then a fixed shuffle tree
-    const int j = threadIdx.x / DOT_G, g = threadIdx.x % DOT_G;
-    double t = 0;
-    if (j < nout) {
-        const int nb = (int)gridDim.x;
-        int b = g;
-        double t1 = 0, t2 = 0, t3 = 0;
-        for (; b + 3 * DOT_G < nb; b += 4 * DOT_G) {
-            t += __ldcg(&part[(size_t)b * nout + j]);
-            t1 += __ldcg(&part[(size_t)(b + DOT_G) * nout + j]);
-            t2 += __ldcg(&part[(size_t)(b + 2 * DOT_G) * nout + j]);
-            t3 += __ldcg(&part[(size_t)(b + 3 * DOT_G) * nout + j]);
-        }
-        for (; b < nb; b += DOT_G) t += __ldcg(&part[(size_t)b * nout + j]);
-        t = (t + t1) + (t2 + t3);
-    }
+    // a warp reads the outputs of one block side by side; warp g takes blocks
+    // g, g + NW, ... with eight loads in flight (one output: a block per thread)
+    constexpr int U = 8;
+    const int j = ONE ? 0 : lane, g = ONE ? (int)threadIdx.x : wp, st = ONE ? NT : NW;
+    double t[U];
 #pragma unroll
-    for (int o = DOT_G / 2; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o, DOT_G);
-    if (j < nout && g == 0) out[j] = t;
-    if (threadIdx.x == 0) *counter = 0;
-}
-
-// v = w * scale[0]; with vk given, v = vbase + (*vk) * n (the next Krylov vector)
-// (16-byte chunks; w and v may be the same vector)
-template <class T>
-__global__ void __launch_bounds__(256) k_imp_scale(const int n, const T* w, const double* __restrict__ scale, T* v,
-                                                   const int* __restrict__ vk, const int* __restrict__ stop) {
-    if (stop && *stop) return;
-    using VT = typename Vec16<T>::type;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (vk) v += (long long)*vk * n;
-    const T sc = (T)scale[0];
-    if (i < n / Vec16<T>::W) {
-        VT a = reinterpret_cast<const VT*>(w)[i];
-        vscale(a, sc);
-        reinterpret_cast<VT*>(v)[i] = a;
+    for (int u = 0; u < U; ++u) t[u] = 0;
+    if (j < nout)
+        for (int b = g; b < nblk; b += U * st)
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (b + u * st < nblk) t[u] += __ldcg(&part[(size_t)(b + u * st) * nout + j]);
+    double v = ((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7]));
+    if (ONE) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if (lane == 0) sh[wp][0] = v;
+    } else {
+        sh[wp][lane] = v;
     }
+    __syncthreads();
+    if (threadIdx.x == 0) *counter = 0;
+    if ((int)threadIdx.x >= nout) return false;
+    double sum = 0;
+#pragma unroll
+    for (int k = 0; k < NW; ++k) sum += sh[k][threadIdx.x];
+    total = sum;
+    return true;
 }
 
-// Arnoldi step j = c->k, classical Gram-Schmidt twice: h1 (first pass) and
-// h2 (second pass) are summed into column j; then the Givens rotations and
-// the residual estimate.  One warp: the column and the rotations are staged
-// in shared memory so the sequential part runs on shared memory, not on
-// dependent global loads.
-__global__ void __launch_bounds__(32) k_imp_arnoldi(GmresCtl* c, const double* __restrict__ h1,
-                                                    const double* __restrict__ h2, const double* __restrict__ ww,
-                                                    double* __restrict__ scale) {
-    __shared__ double col[GM_M + 1], cs[GM_M], sn[GM_M], gj[1];
-    const int lane = threadIdx.x;
-    if (c->stop) {
-        if (lane == 0 && c->graph) cudaGraphSetConditional(c->hin, 0);
+// givens (MODE 2 of an Arnoldi step, else null): the control block whose
+// column the step completes, with h1 and hin = h2; scale: 1/||w||
+template <class T, int MODE>
+__global__ void __launch_bounds__(DOT_THREADS, MODE == 1 ? 1 : 2)
+    k_imp_dots(const int n, int nv, const int* __restrict__ nvk, const T* __restrict__ V, T* w,
+               const double* __restrict__ hin, double* __restrict__ part, unsigned* __restrict__ counter,
+               double* __restrict__ out, const int* stop, GmresCtl* givens, const double* __restrict__ h1,
+               double* __restrict__ scale) {
+    __shared__ T hs[GM_M + 2];
+    __shared__ GivensCol gc;
+    if (stop && *stop) {
+        // an Arnoldi step launched after the cycle's end
+        if (MODE == 2 && givens && givens->graph && blockIdx.x == 0 && threadIdx.x == 0)
+            cudaGraphSetConditional(givens->hin, 0);
         return;
     }
-    const int j = c->k;
-    for (int t = lane; t <= j; t += 32) col[t] = h1[t] + h2[t];
-    for (int t = lane; t < j; t += 32) {
-        cs[t] = c->cs[t];
-        sn[t] = c->sn[t];
-    }
-    if (lane == 0) gj[0] = c->g[j];
-    __syncwarp();
-    if (lane == 0) {
-        const double hn = sqrt(fmax(ww[0], 0.0));
-        col[j + 1] = hn;
-        c->hnext = hn;
-        scale[0] = hn > 0 ? 1.0 / hn : 0.0;
-        for (int i = 0; i < j; ++i) {
-            const double a = col[i], b = col[i + 1];
-            col[i] = cs[i] * a + sn[i] * b;
-            col[i + 1] = -sn[i] * a + cs[i] * b;
+    if (nvk) nv = *nvk + 1;  // v_0 .. v_k of the current Arnoldi step
+    const int nout = MODE == 2 ? 1 : nv;
+    // block 0 of an Arnoldi step's MODE 2 sees to the column, the others sum
+    const int first = MODE == 2 && givens ? 1 : 0, blk = (int)blockIdx.x - first, nblk = (int)gridDim.x - first;
+    const bool adds = blk >= 0;
+    T acc[GM_M + 2];
+#pragma unroll
+    for (int j = 0; j < GM_M + 2; ++j) acc[j] = 0;
+    if (!adds) {
+        if (threadIdx.x < 32) {
+            givens_column(givens, h1, hin, gc);
+            __threadfence();  // the column is visible before the block is counted
         }
-        const double a = col[j], b = col[j + 1];
-        const double r = sqrt(a * a + b * b);
-        const double cj = r > 0 ? a / r : 1.0, sj = r > 0 ? b / r : 0.0;
-        c->cs[j] = cj;
-        c->sn[j] = sj;
-        col[j] = r;
-        col[j + 1] = 0;
-        const double g = gj[0];
-        c->g[j + 1] = -sj * g;
-        c->g[j] = cj * g;
-        c->res = fabs(sj * g);
-        c->k = j + 1;
-        c->iters += 1;
-        const int st = (c->res <= c->tol || j + 1 == GM_M || hn == 0 || c->iters >= c->max_iters) ? 1 : 0;
-        c->stop = st;
-        if (c->graph) cudaGraphSetConditional(c->hin, st ? 0 : 1);
+    } else {
+        if (threadIdx.x < GM_M + 2) hs[threadIdx.x] = (int)threadIdx.x < nv ? (T)hin[threadIdx.x] : T(0);
+        __syncthreads();
+        // per-thread partial sums in T over 16-byte chunks of the vectors (a few
+        // chunks each; n is 4 * cells, so whole chunks)
+        using VT = typename Vec16<T>::type;
+        const int nc = n / Vec16<T>::W;
+        const VT* __restrict__ Vv = reinterpret_cast<const VT*>(V);
+        VT* wv = reinterpret_cast<VT*>(w);
+        for (int i = blk * blockDim.x + threadIdx.x; i < nc; i += nblk * blockDim.x) {
+            VT wi = wv[i];
+            if (MODE == 1) {
+                // the basis chunks stay in registers for the second product
+                // (one block per SM; the loads of a chunk are all in flight at
+                // once)
+                VT vv[GM_M + 1];
+#pragma unroll
+                for (int j0 = 0; j0 <= GM_M; j0 += DOT_U)
+                    if (j0 < nv)
+#pragma unroll
+                        for (int j = j0; j < j0 + DOT_U && j <= GM_M; ++j)
+                            vv[j] = j < nv ? Vv[(size_t)j * nc + i] : VT();
+#pragma unroll
+                for (int j0 = 0; j0 <= GM_M; j0 += DOT_U)
+                    if (j0 < nv)
+#pragma unroll
+                        for (int j = j0; j < j0 + DOT_U && j <= GM_M; ++j) vsub(wi, hs[j], vv[j]);
+                wv[i] = wi;
+#pragma unroll
+                for (int j0 = 0; j0 <= GM_M; j0 += DOT_U)
+                    if (j0 < nv)
+#pragma unroll
+                        for (int j = j0; j < j0 + DOT_U && j <= GM_M; ++j) acc[j] += vdot(vv[j], wi);
+            } else {
+#pragma unroll
+                for (int j0 = 0; j0 <= GM_M; j0 += DOT_U)
+                    if (j0 < nv) {
+                        VT vv[DOT_U];
+#pragma unroll
+                        for (int u = 0; u < DOT_U; ++u)
+                            vv[u] = j0 + u < nv ? Vv[(size_t)(j0 + u) * nc + i] : VT();
+#pragma unroll
+                        for (int u = 0; u < DOT_U; ++u) vsub(wi, hs[j0 + u], vv[u]);
+                    }
+                if (nv > 0) wv[i] = wi;
+                acc[0] += vdot(wi, wi);
+            }
+        }
     }
-    __syncwarp();
-    for (int t = lane; t <= j + 1; t += 32) c->H[t + (GM_M + 1) * j] = col[t];
+    double t;
+    if (grid_sums<T, DOT_THREADS, MODE == 2>(acc, nout, blk, nblk, part, counter, t)) {
+        out[threadIdx.x] = t;
+        if (MODE == 2 && givens) givens_finish(givens, t, scale);
+    }
 }
 
-// Back substitution R y = g over the k steps of the cycle (one warp; the
-// triangle is staged in shared memory)
-__global__ void __launch_bounds__(32) k_imp_solve_y(GmresCtl* c) {
-    __shared__ double R[GM_M * GM_M], g[GM_M], y[GM_M];
-    const int k = c->k;
-    for (int t = threadIdx.x; t < k * k; t += 32) {
-        const int i = t % k, l = t / k;
-        R[i + GM_M * l] = c->H[i + (GM_M + 1) * l];
+// w = M x and out_j = v_j . w, j <= *vk, in one pass over the rows: the
+// product's row is in registers when the basis is read, and one launch and one
+// pass over w less per Arnoldi step.
+template <class T, int RT>
+__global__ void __launch_bounds__(DOT_THREADS, 2)
+    k_imp_spmv_dots(const int n_rows, const Ell e, const T* __restrict__ dblk, const T* __restrict__ off,
+                    const T* __restrict__ x, T* __restrict__ w, const int* __restrict__ vk, const T* __restrict__ V,
+                    double* __restrict__ part, unsigned* __restrict__ counter, double* __restrict__ out,
+                    const int* __restrict__ stop, const int* __restrict__ case_done) {
+    constexpr int NC = 4 / RT;
+    if (*stop) return;
+    const int nv = *vk + 1;
+    T acc[GM_M + 2];
+#pragma unroll
+    for (int j = 0; j < GM_M + 2; ++j) acc[j] = 0;
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < RT * (long long)n_rows;
+         t += (long long)gridDim.x * blockDim.x) {
+        const int p = (int)(t / RT), c = NC * (int)(t % RT);
+        T y[NC];
+#pragma unroll
+        for (int r = 0; r < NC; ++r) y[r] = T(0);
+        if (!held(e.case_row, case_done, p)) spmv_row<T, RT>(n_rows, e, dblk, off, x, p, c, y);
+        row_store<T, RT>(w, p, c, y);
+#pragma unroll
+        for (int j0 = 0; j0 <= GM_M; j0 += DOT_U)
+            if (j0 < nv) {
+                T v[DOT_U][NC];
+#pragma unroll
+                for (int u = 0; u < DOT_U; ++u) {
+#pragma unroll
+                    for (int r = 0; r < NC; ++r) v[u][r] = T(0);
+                    if (j0 + u < nv) row_load<T, RT>(V + (size_t)(j0 + u) * 4 * n_rows, p, c, v[u]);
+                }
+#pragma unroll
+                for (int u = 0; u < DOT_U; ++u) {
+                    if constexpr (NC == 1) acc[j0 + u] += v[u][0] * y[0];
+                    else acc[j0 + u] += ((v[u][0] * y[0] + v[u][1] * y[1]) + v[u][2] * y[2]) + v[u][3] * y[3];
+                }
+            }
     }
-    for (int t = threadIdx.x; t < k; t += 32) g[t] = c->g[t];
+    double s;
+    if (grid_sums<T, DOT_THREADS, false>(acc, nv, (int)blockIdx.x, (int)gridDim.x, part, counter, s)) out[threadIdx.x] = s;
+}
+
+// Back substitution R y = g over the k steps of the cycle: one warp, a lane
+// per unknown, each solved unknown's column taken off the lanes that still
+// wait (the triangle is staged in shared memory).
+__global__ void __launch_bounds__(32) k_imp_solve_y(GmresCtl* c) {
+    __shared__ double R[GM_M * GM_M];
+    const int k = c->k, i = threadIdx.x;
+    for (int t = i; t < k * k; t += 32) {
+        const int r = t % k, l = t / k;
+        R[r + GM_M * l] = c->H[r + (GM_M + 1) * l];
+    }
+    double g = i < k ? c->g[i] : 0.0;
     __syncwarp();
-    if (threadIdx.x == 0)
-        for (int i = k - 1; i >= 0; --i) {
-            double s = g[i];
-            for (int l = i + 1; l < k; ++l) s -= R[i + GM_M * l] * y[l];
-            const double d = R[i + GM_M * i];
-            y[i] = d != 0 ? s / d : 0.0;
+    const double d = i < k ? R[i + GM_M * i] : 0.0;
+    const double inv = d != 0 ? 1.0 / d : 0.0;
+    for (int l = k - 1; l >= 0; --l) {
+        if (i == l) {  // g / d: the product with 1/d and one correction
+            const double y = g * inv;
+            g = fma(fma(-y, d, g), inv, y);
         }
-    __syncwarp();
-    for (int t = threadIdx.x; t < k; t += 32) c->y[t] = y[t];
+        const double yl = __shfl_sync(0xffffffffu, g, l);
+        if (i < l) g -= R[i + GM_M * l] * yl;
+    }
+    if (i < k) c->y[i] = g;
 }
 
 // t = sum_j y_j v_j over the k steps
@@ -1008,8 +1193,11 @@ ImplicitEngine* implicit_create(const StepArgs& a, bool f32, bool graph, const s
     int dev_id = 0, sms = 0;
     cudaGetDevice(&dev_id);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_id);
-    // two resident blocks per SM at most: the last block then sums few partials
-    e->nbd = std::max(1, std::min(2 * std::max(sms, 1), nb_(e->n4, dev::DOT_THREADS * 4)));
+    // one 16-byte chunk per thread until every SM holds two blocks (more would
+    // leave the last block too many partial sums); a system of 16k rows in
+    // FP64 ran on 64 blocks with two chunks per thread before
+    const int chunks = (int)(((size_t)e->n4 * e->ts()) / 16);
+    e->nbd = std::max(1, std::min(2 * std::max(sms, 1), nb_(chunks, dev::DOT_THREADS)));
     e->nbd1 = std::max(1, std::min(std::max(sms, 1), e->nbd));
     chk(cudaMalloc((void**)&e->part, (size_t)e->nbd * (dev::GM_M + 1) * 8));
     chk(cudaMalloc((void**)&e->small, (2 * (dev::GM_M + 1) + 2) * 8));
@@ -1097,45 +1285,92 @@ struct Ops {
     const StepArgs& a;
     cudaStream_t s;
     dev::KM<double> m;
-    using V4 = typename dev::B4<T>::type;
     Ops(ImplicitEngine* e_, const StepArgs& a_, cudaStream_t s_) : e(e_), a(a_), s(s_), m(dev::make_km<double>(a_)) {}
     T* vec(int j) const { return (T*)e->V + (size_t)j * e->n4; }
     int* stop() const { return &e->ctl->stop; }
     void spmv(const T* x, T* y, const int* st) const {
-        dev::k_imp_spmv<T><<<nb_(e->N, 256), 256, 0, s>>>(e->N, e->ell(), (const T*)e->dblk, (const T*)e->off,
-                                                          (const V4*)x, (V4*)y, st, a.case_done);
+        dev::k_imp_spmv<T><<<nb_(e->N, 256), 256, 0, s>>>(e->N, e->ell(), (const T*)e->dblk, (const T*)e->off, x, y,
+                                                          st, a.case_done);
     }
     // t = b in row order
     void gather_b(const double* b, T* t) const {
         dev::k_imp_gather_b<T><<<nb_(e->n4, 256), 256, 0, s>>>(e->n4, b, e->perm, t);
     }
+    // four threads per row for a launch over n rows?
+    // (measured, whole implicit iteration: FP64 16k rows 60.3 ms with one thread
+    // per row always, 44.9 ms with four; FP32 131k rows 17.6 ms with one always,
+    // 19.4 ms with four always, 16.9 ms with four below 40,000 rows)
+    static bool four(long long n) { return n < 40000; }
     // one symmetric multicolour block Gauss-Seidel sweep from x = 0 (the
     // ILU(0) factors in the colour ordering); the input is r, or the current
     // Krylov vector V + k*n when rk is given.  The forward sweep forms every
-    // cell (reading lower colours only); the backward sweep skips the top
-    // colour, whose value it would form again unchanged.
-    void precond(const T* r, const int* rk, T* x, const int* st) const {
+    // cell (reading lower colours only) from colour `first` on; the backward
+    // sweep skips the top colour, whose value it would form again unchanged.
+    void precond(const T* r, const int* rk, T* x, const int* st, int first = 0) const {
         const int C = e->n_colors;
-        for (int k = 0; k < 2 * C - 1; ++k) {
+        for (int k = first; k < 2 * C - 1; ++k) {
             const int c = k < C ? k : 2 * C - 2 - k;
             const int c0 = e->color_ptr[c], cn = e->color_ptr[c + 1] - c0;
             if (cn == 0) continue;
-            dev::k_imp_gs<T><<<nb_(cn, 256), 256, 0, s>>>(e->ell(), e->N, (const T*)e->dinv, (const T*)e->off, c0,
-                                                          cn, r, rk, (long long)e->n4, (V4*)x, st, a.case_done,
-                                                          k < C);
+            if (four(cn))
+                dev::k_imp_gs<T, 4><<<nb_(4LL * cn, 128), 128, 0, s>>>(e->ell(), e->N, (const T*)e->dinv,
+                                                                       (const T*)e->off, c0, cn, r, rk,
+                                                                       (long long)e->n4, x, st, a.case_done, k < C);
+            else
+                dev::k_imp_gs<T, 1><<<nb_(cn, 128), 128, 0, s>>>(e->ell(), e->N, (const T*)e->dinv, (const T*)e->off,
+                                                                 c0, cn, r, rk, (long long)e->n4, x, st, a.case_done,
+                                                                 k < C);
         }
     }
-    // MODE 0: out = V^T w; 1: w -= V hin, out = V^T w; 2: w -= V hin, out = w.w
+    // v_k = w * scale, x = P^-1 v_k (the first colour with the scaling)
+    void scale_precond(const T* w, const double* sc, T* V, const int* k, T* x, const int* st) const {
+        if (four(e->N))
+            dev::k_imp_scale_gs<T, 4><<<nb_(e->n4, 128), 128, 0, s>>>(e->ell(), e->N, (const T*)e->dinv,
+                                                                      e->color_ptr[1], w, sc, V, k, x, st,
+                                                                      a.case_done);
+        else
+            dev::k_imp_scale_gs<T, 1><<<nb_(e->N, 128), 128, 0, s>>>(e->ell(), e->N, (const T*)e->dinv,
+                                                                     e->color_ptr[1], w, sc, V, k, x, st,
+                                                                     a.case_done);
+        precond(V, k, x, st, 1);
+    }
+    // MODE 1: w -= V hin, out = V^T w; 2: w -= V hin, out = w.w
     template <int MODE>
     void dots(int nv, const int* nvk, const T* V, T* w, const double* hin, double* out, const int* st) const {
         // MODE 1 holds one block per SM
         const int g = MODE == 1 ? e->nbd1 : e->nbd;
         dev::k_imp_dots<T, MODE><<<g, dev::DOT_THREADS, 0, s>>>(e->n4, nv, nvk, V, w, hin, e->part, e->counter, out,
-                                                              st);
+                                                              st, nullptr, nullptr, nullptr);
     }
-    // v = w * scale (k given: v = V_{*k})
-    void scale(const T* w, const double* sc, T* v, const int* k, const int* st) const {
-        dev::k_imp_scale<T><<<nb_(e->n4 / (16 / (int)sizeof(T)), 256), 256, 0, s>>>(e->n4, w, sc, v, k, st);
+    // w = M x, out = V^T w
+    void spmv_dots(const T* x, T* w, const int* k, const T* V, double* out, const int* st) const {
+        if (four(e->N))
+            dev::k_imp_spmv_dots<T, 4><<<e->nbd, dev::DOT_THREADS, 0, s>>>(
+                e->N, e->ell(), (const T*)e->dblk, (const T*)e->off, x, w, k, V, e->part, e->counter, out, st,
+                a.case_done);
+        else
+            dev::k_imp_spmv_dots<T, 1><<<e->nbd, dev::DOT_THREADS, 0, s>>>(
+                e->N, e->ell(), (const T*)e->dblk, (const T*)e->off, x, w, k, V, e->part, e->counter, out, st,
+                a.case_done);
+    }
+    // the end of an Arnoldi step: MODE 2 and column k of the Hessenberg matrix
+    // (a block of its own for the earlier rotations, inside the one wave that
+    // two blocks per SM make: a 305th block would wait for another to end)
+    void finish_step(const int* k, const T* V, T* w, const double* h1, const double* h2, double* ww, double* sc,
+                     const int* st) const {
+        const int g = std::max(2, std::min(e->nbd + 1, 2 * e->nbd1));
+        dev::k_imp_dots<T, 2><<<g, dev::DOT_THREADS, 0, s>>>(e->n4, 0, k, V, w, h2, e->part, e->counter, ww, st,
+                                                           e->ctl, h1, sc);
+    }
+    // Arnoldi step k: v_k = w * scale, z = P^-1 v_k, w = M z, CGS2 against
+    // v_0..v_k in three passes over the basis (h1 = V^T w; w -= V h1 and
+    // h2 = V^T w; w -= V h2 and ||w||^2), rotations
+    void arnoldi_step(T* V, T* w, T* z, double* h1, double* h2, double* ww, double* sc, const int* k,
+                      const int* st) const {
+        scale_precond(w, sc, V, k, z, st);
+        spmv_dots(z, w, k, V, h1, st);
+        dots<1>(0, k, V, w, h1, h2, st);
+        finish_step(k, V, w, h1, h2, ww, sc, st);
     }
 };
 
@@ -1185,12 +1420,11 @@ cudaGraphExec_t build_gmres_graph(ImplicitEngine* e, const Ops<T>& o0, const dou
     // main graph: first cycle set-up, the restart loop, the control block back to the host
     chk(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     Ops<T> o(e, o0.a, s);
-    T* v0 = o.vec(0);
+    T* w = (T*)e->w;  // the vector that becomes v_0 (scaled by the first Arnoldi step)
     cudaMemsetAsync(e->x, 0, (size_t)n * 8, s);
-    o.gather_b(b, v0);
-    o.template dots<0>(1, nullptr, v0, v0, nullptr, ww, nullptr);
+    o.gather_b(b, w);
+    o.template dots<2>(0, nullptr, nullptr, w, nullptr, ww, nullptr);
     k_imp_cycle_init<<<1, 1, 0, s>>>(e->ctl, ww, scale, 1, 1e-2, max_iters);
-    o.scale(v0, scale, v0, nullptr, stop);
     cudaGraph_t body_out = add_while(s, &hout);
     cudaMemcpyAsync(e->h_ctl, e->ctl, sizeof(GmresCtl), cudaMemcpyDeviceToHost, s);
     cudaGraph_t G;
@@ -1207,24 +1441,14 @@ cudaGraphExec_t build_gmres_graph(ImplicitEngine* e, const Ops<T>& o0, const dou
         k_imp_addx<T><<<nb_(n, 256), 256, 0, s2>>>(n, (const T*)e->z, e->x);
         k_imp_outer_check<<<1, 1, 0, s2>>>(e->ctl);
         k_imp_cast<T><<<nb_(n, 256), 256, 0, s2>>>(n, e->x, (T*)e->t, halt);
-        q.spmv((const T*)e->t, (T*)e->w, halt);
-        k_imp_resid<T><<<nb_(n, 256), 256, 0, s2>>>(n, b, e->perm, (const T*)e->w, q.vec(0), halt);
-        q.template dots<0>(1, nullptr, q.vec(0), q.vec(0), nullptr, ww, halt);
+        q.spmv((const T*)e->t, (T*)e->z, halt);
+        k_imp_resid<T><<<nb_(n, 256), 256, 0, s2>>>(n, b, e->perm, (const T*)e->z, w, halt);
+        q.template dots<2>(0, nullptr, nullptr, w, nullptr, ww, halt);
         k_imp_cycle_init<<<1, 1, 0, s2>>>(e->ctl, ww, scale, 0, 1e-2, max_iters);
-        q.scale(q.vec(0), scale, q.vec(0), nullptr, halt);
         chk(cudaStreamEndCapture(s2, &body_out));
-        // Arnoldi step k: z = P^-1 v_k, w = M z, CGS2 against v_0..v_k, rotations, v_{k+1}
         chk(cudaStreamBeginCaptureToGraph(s3, body_in, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
         Ops<T> r(e, o0.a, s3);
-        r.precond(r.vec(0), kptr, (T*)e->z, stop);
-        r.spmv((const T*)e->z, (T*)e->w, stop);
-        // CGS2 in three passes over the basis: h1 = V^T w; w -= V h1 and
-        // h2 = V^T w; w -= V h2 and ||w||^2
-        r.template dots<0>(0, kptr, r.vec(0), (T*)e->w, nullptr, h1, stop);
-        r.template dots<1>(0, kptr, r.vec(0), (T*)e->w, h1, h2, stop);
-        r.template dots<2>(0, kptr, r.vec(0), (T*)e->w, h2, ww, stop);
-        k_imp_arnoldi<<<1, 32, 0, s3>>>(e->ctl, h1, h2, ww, scale);
-        r.scale((const T*)e->w, scale, r.vec(0), kptr, stop);
+        r.arnoldi_step(r.vec(0), w, (T*)e->z, h1, h2, ww, scale, kptr, stop);
         chk(cudaStreamEndCapture(s3, &body_in));
     }
     cudaGraphExec_t ex;
@@ -1260,25 +1484,18 @@ int gmres_host_loop(ImplicitEngine* e, const StepArgs& a, const double* b, cudaS
             cudaStreamSynchronize(s) != cudaSuccess)
             throw Error(7, "implicit solver: GMRES failed");
     };
-    T* v0 = o.vec(0);
+    T* w = (T*)e->w;
     cudaMemsetAsync(e->x, 0, (size_t)n * 8, s);
-    o.gather_b(b, v0);
-    o.template dots<0>(1, nullptr, v0, v0, nullptr, ww, nullptr);
+    o.gather_b(b, w);
+    o.template dots<2>(0, nullptr, nullptr, w, nullptr, ww, nullptr);
     k_imp_cycle_init<<<1, 1, 0, s>>>(e->ctl, ww, scale, 1, 1e-2, max_iters);
-    o.scale(v0, scale, v0, nullptr, stop);
     read_ctl();
     if (!e->h_ctl->stop) {
         for (;;) {
             for (;;) {  // Arnoldi steps of the cycle
                 read_ctl();
                 if (e->h_ctl->stop) break;
-                o.precond(o.vec(0), kptr, (T*)e->z, stop);
-                o.spmv((const T*)e->z, (T*)e->w, stop);
-                o.template dots<0>(0, kptr, o.vec(0), (T*)e->w, nullptr, h1, stop);
-                o.template dots<1>(0, kptr, o.vec(0), (T*)e->w, h1, h2, stop);
-                o.template dots<2>(0, kptr, o.vec(0), (T*)e->w, h2, ww, stop);
-                k_imp_arnoldi<<<1, 32, 0, s>>>(e->ctl, h1, h2, ww, scale);
-                o.scale((const T*)e->w, scale, o.vec(0), kptr, stop);
+                o.arnoldi_step(o.vec(0), w, (T*)e->z, h1, h2, ww, scale, kptr, stop);
             }
             k_imp_solve_y<<<1, 32, 0, s>>>(e->ctl);
             k_imp_lincomb<T><<<nb_(n, 256), 256, 0, s>>>(n, o.vec(0), e->ctl, (T*)e->t);
@@ -1286,11 +1503,10 @@ int gmres_host_loop(ImplicitEngine* e, const StepArgs& a, const double* b, cudaS
             k_imp_addx<T><<<nb_(n, 256), 256, 0, s>>>(n, (const T*)e->z, e->x);
             k_imp_outer_check<<<1, 1, 0, s>>>(e->ctl);
             k_imp_cast<T><<<nb_(n, 256), 256, 0, s>>>(n, e->x, (T*)e->t, halt);
-            o.spmv((const T*)e->t, (T*)e->w, halt);
-            k_imp_resid<T><<<nb_(n, 256), 256, 0, s>>>(n, b, e->perm, (const T*)e->w, o.vec(0), halt);
-            o.template dots<0>(1, nullptr, o.vec(0), o.vec(0), nullptr, ww, halt);
+            o.spmv((const T*)e->t, (T*)e->z, halt);
+            k_imp_resid<T><<<nb_(n, 256), 256, 0, s>>>(n, b, e->perm, (const T*)e->z, w, halt);
+            o.template dots<2>(0, nullptr, nullptr, w, nullptr, ww, halt);
             k_imp_cycle_init<<<1, 1, 0, s>>>(e->ctl, ww, scale, 0, 1e-2, max_iters);
-            o.scale(o.vec(0), scale, o.vec(0), nullptr, halt);
             read_ctl();
             if (e->h_ctl->halt) break;
         }
