@@ -37,6 +37,7 @@
 
 #include "afx_host.hpp"
 #include "afx_kernels_impl.cuh"
+#include "afx_pdl.cuh"
 
 namespace afx {
 namespace dev {
@@ -66,38 +67,37 @@ template <> struct B4<float> { using type = float4; };
 // Krylov-side vectors in their own precision T: FP32 arithmetic stays in the
 // FP32 pipes (a float-to-double conversion per operand would run on GB300's
 // FP64 pipe, at ~1/64 of the FP32 rate)
-__device__ __forceinline__ void ldt(const d4* p, double* v) { ld4(p, v); }
+__device__ __forceinline__ void ldt(const d4* p, double* v) {
+    const double2* c = reinterpret_cast<const double2*>(p);
+    const double2 a = ldw(c), b = ldw(c + 1);
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
 __device__ __forceinline__ void ldt(const float4* p, float* v) {
-    const float4 a = *p;
+    const float4 a = ldw(p);
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
 }
 __device__ __forceinline__ void stt(d4* p, const double* v) { st4(p, v); }
 __device__ __forceinline__ void stt(float4* p, const float* v) { *p = make_float4(v[0], v[1], v[2], v[3]); }
 
-// Row r of a 4x4 block (row-major) times x: the row is one (FP32) or two
-// (FP64) 16-byte chunks, `stride` chunks apart.
-template <class T>
-__device__ __forceinline__ T row_dot(const T* __restrict__ chunk, const size_t stride, const T* x);
-template <>
-__device__ __forceinline__ float row_dot<float>(const float* __restrict__ chunk, const size_t, const float* x) {
-    const float4 a = __ldg(reinterpret_cast<const float4*>(chunk));
-    float t = 0;
-    t += a.x * x[0];
-    t += a.y * x[1];
-    t += a.z * x[2];
-    t += a.w * x[3];
-    return t;
+// Row r of a 4x4 block (row-major), one (FP32) or two (FP64) 16-byte chunks
+// `stride` chunks apart, and its product with x.
+template <class T> struct Row { T a[4]; };
+__device__ __forceinline__ Row<float> row_at(const float* __restrict__ chunk, const size_t) {
+    const float4 v = __ldg(reinterpret_cast<const float4*>(chunk));
+    return Row<float>{{v.x, v.y, v.z, v.w}};
 }
-template <>
-__device__ __forceinline__ double row_dot<double>(const double* __restrict__ chunk, const size_t stride,
-                                                  const double* x) {
+__device__ __forceinline__ Row<double> row_at(const double* __restrict__ chunk, const size_t stride) {
     const double2* c = reinterpret_cast<const double2*>(chunk);
     const double2 u = __ldg(c), v = __ldg(c + stride);
-    double t = 0;
-    t += u.x * x[0];
-    t += u.y * x[1];
-    t += v.x * x[2];
-    t += v.y * x[3];
+    return Row<double>{{u.x, u.y, v.x, v.y}};
+}
+template <class T>
+__device__ __forceinline__ T row_dot(const Row<T>& r, const T* x) {
+    T t = 0;
+    t += r.a[0] * x[0];
+    t += r.a[1] * x[1];
+    t += r.a[2] * x[2];
+    t += r.a[3] * x[3];
     return t;
 }
 
@@ -221,12 +221,12 @@ __device__ __forceinline__ size_t ell_at(const int N, const int p, const int s, 
     constexpr int W = Ell16<T>::W, CPB = Ell16<T>::CPB;
     return ((size_t)(s * CPB + k / W) * N + p) * W + (k % W);
 }
-// row r of the block of slot s of row p, times x
+// row r of the block of slot s of row p
 template <class T>
-__device__ __forceinline__ T ell_row(const T* __restrict__ off, const int N, const int p, const int s, const int r,
-                                     const T* x) {
+__device__ __forceinline__ Row<T> ell_row(const T* __restrict__ off, const int N, const int p, const int s,
+                                          const int r) {
     constexpr int W = Ell16<T>::W, CPB = Ell16<T>::CPB;
-    return row_dot<T>(off + ((size_t)(s * CPB + r * (CPB / 4)) * N + p) * W, (size_t)N, x);
+    return row_at(off + ((size_t)(s * CPB + r * (CPB / 4)) * N + p) * W, (size_t)N);
 }
 
 // Diagonal block A/dt I + sum (own: J, other: -K) of row p and its inverse
@@ -448,10 +448,15 @@ __global__ void __launch_bounds__(128) k_imp_ilu(const Ell e, const int N, const
 // The sums run in the order of the block form either way, so the results do
 // not depend on RT.  Bound by latency at these sizes: a colour of 3,300 rows in
 // FP64 took 8.0 us with one thread per row in blocks of 256, 3.8 us with four.
+// Matrix data is read before pdl_wait() where it fits in registers (AHEAD):
+// the next colour's blocks arrive while the previous colour is computed, and
+// only the gathers of x remain after the wait.
+template <class T, int RT> constexpr bool AHEAD = RT == 4 || sizeof(T) == 4;
+
 template <class T, int RT>
-__device__ __forceinline__ void row_load(const T* __restrict__ r, const size_t p, const int c, T* s) {
+__device__ __forceinline__ void row_load(const T* r, const size_t p, const int c, T* s) {
     if constexpr (RT == 1) ldt(reinterpret_cast<const typename B4<T>::type*>(r) + p, s);
-    else s[0] = r[4 * p + c];
+    else s[0] = ldw(r + 4 * p + c);
 }
 template <class T, int RT>
 __device__ __forceinline__ void row_store(T* r, const size_t p, const int c, const T* s) {
@@ -459,18 +464,16 @@ __device__ __forceinline__ void row_store(T* r, const size_t p, const int c, con
     else r[4 * p + c] = s[0];
 }
 
-// rows of M x for row p
+// rows of M x for row p (the diagonal block's rows already in d)
 template <class T, int RT>
-__device__ __forceinline__ void spmv_row(const int n_rows, const Ell& e, const T* __restrict__ dblk,
-                                         const T* __restrict__ off, const T* __restrict__ x, const int p, const int c,
-                                         T* y) {
+__device__ __forceinline__ void spmv_row(const int n_rows, const int4 col, const Row<T>* d, const T* __restrict__ off,
+                                         const T* x, const int p, const int c, T* y) {
     constexpr int NC = 4 / RT;
     const typename B4<T>::type* x4 = reinterpret_cast<const typename B4<T>::type*>(x);
     T xi[4];
     ldt(&x4[p], xi);
-    const int4 col = __ldg(&e.col[p]);
 #pragma unroll
-    for (int r = 0; r < NC; ++r) y[r] = row_dot<T>(dblk + 16 * (size_t)p + 4 * (c + r), 1, xi);
+    for (int r = 0; r < NC; ++r) y[r] = row_dot<T>(d[r], xi);
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
         const int q = pick(col, s);
@@ -478,28 +481,37 @@ __device__ __forceinline__ void spmv_row(const int n_rows, const Ell& e, const T
         T xo[4];
         ldt(&x4[q], xo);
 #pragma unroll
-        for (int r = 0; r < NC; ++r) y[r] += ell_row<T>(off, n_rows, p, s, c + r, xo);
+        for (int r = 0; r < NC; ++r) y[r] += row_dot<T>(ell_row<T>(off, n_rows, p, s, c + r), xo);
     }
+}
+template <class T, int RT>
+__device__ __forceinline__ void diag_rows(const T* __restrict__ d, const int p, const int c, Row<T>* o) {
+#pragma unroll
+    for (int r = 0; r < 4 / RT; ++r) o[r] = row_at(d + 16 * (size_t)p + 4 * (c + r), 1);
 }
 
 // y = M x over the rows (diagonal block, then the slots in face order)
 template <class T>
 __global__ void __launch_bounds__(256) k_imp_spmv(const int n_rows, const Ell e, const T* __restrict__ dblk,
-                                                  const T* __restrict__ off, const T* __restrict__ x,
-                                                  T* __restrict__ y, const int* __restrict__ stop,
+                                                  const T* __restrict__ off, const T* x, T* y, const int* stop,
                                                   const int* __restrict__ case_done) {
-    if (stop && *stop) return;
+    pdl_wait();
+    if (stop && ldw(stop)) return;
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n_rows) return;
     T yr[4] = {0, 0, 0, 0};
-    if (!held(e.case_row, case_done, p)) spmv_row<T, 1>(n_rows, e, dblk, off, x, p, 0, yr);
+    if (!held(e.case_row, case_done, p)) {
+        Row<T> d[4];
+        diag_rows<T, 1>(dblk, p, 0, d);
+        spmv_row<T, 1>(n_rows, __ldg(&e.col[p]), d, off, x, p, 0, yr);
+    }
     row_store<T, 1>(y, p, 0, yr);
 }
 
-// Rows of D_p^-1 s; with RT = 4 the row's four threads hold one component of s each
+// Rows of D_p^-1 s (its rows in d); with RT = 4 the row's four threads hold one
+// component of s each
 template <class T, int RT>
-__device__ __forceinline__ void dinv_row(const T* __restrict__ dinv, const int p, const int c, const T* s, T* x) {
-    constexpr int NC = 4 / RT;
+__device__ __forceinline__ void dinv_row(const Row<T>* d, const T* s, T* x) {
     T sv[4];
     if constexpr (RT == 1) {
 #pragma unroll
@@ -510,7 +522,7 @@ __device__ __forceinline__ void dinv_row(const T* __restrict__ dinv, const int p
         for (int k = 0; k < 4; ++k) sv[k] = __shfl_sync(lanes, s[0], k, RT);
     }
 #pragma unroll
-    for (int r = 0; r < NC; ++r) x[r] = row_dot<T>(dinv + 16 * (size_t)p + 4 * (c + r), 1, sv);
+    for (int r = 0; r < 4 / RT; ++r) x[r] = row_dot<T>(d[r], sv);
 }
 
 // One colour (rows c0 .. c0+n-1) of a block Gauss-Seidel sweep:
@@ -520,16 +532,36 @@ __device__ __forceinline__ void dinv_row(const T* __restrict__ dinv, const int p
 // (zero start).
 template <class T, int RT>
 __global__ void __launch_bounds__(128) k_imp_gs(const Ell e, const int N, const T* __restrict__ dinv,
-                                                const T* __restrict__ off, const int c0, const int n,
-                                                const T* __restrict__ rbase, const int* __restrict__ rk,
-                                                const long long stride, T* x, const int* __restrict__ stop,
+                                                const T* __restrict__ off, const int c0, const int n, const T* rbase,
+                                                const int* rk, const long long stride, T* x, const int* stop,
                                                 const int* __restrict__ case_done, const bool fwd) {
     constexpr int NC = 4 / RT;
-    if (stop && *stop) return;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n * RT) return;
-    const T* r = rbase + (rk ? (long long)*rk * stride : 0);
+    const bool in = t < n * RT;
     const int p = c0 + t / RT, c = NC * (t % RT);
+    int4 col = make_int4(-1, -1, -1, -1);
+    Row<T> d[NC], o[4][NC];
+    auto blocks = [&]() {
+        diag_rows<T, RT>(dinv, p, c, d);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (pick(col, k) >= 0)
+#pragma unroll
+                for (int j = 0; j < NC; ++j) o[k][j] = ell_row<T>(off, N, p, k, c + j);
+    };
+    if (in) {
+        col = __ldg(&e.col[p]);
+        if (fwd) {
+            if (col.x >= c0) col.x = -1;
+            if (col.y >= c0) col.y = -1;
+            if (col.z >= c0) col.z = -1;
+            if (col.w >= c0) col.w = -1;
+        }
+        if (AHEAD<T, RT>) blocks();
+    }
+    pdl_wait();
+    if (!in || (stop && ldw(stop))) return;
+    if (!AHEAD<T, RT>) blocks();
     T xr[NC];
     if (held(e.case_row, case_done, p)) {
 #pragma unroll
@@ -538,18 +570,17 @@ __global__ void __launch_bounds__(128) k_imp_gs(const Ell e, const int N, const 
         return;
     }
     T s[NC];
-    row_load<T, RT>(r, p, c, s);
-    const int4 col = __ldg(&e.col[p]);
+    row_load<T, RT>(rbase + (rk ? (long long)ldw(rk) * stride : 0), p, c, s);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const int q = pick(col, k);
-        if (q < 0 || (fwd && q >= c0)) continue;
+        if (q < 0) continue;
         T xo[4];
         ldt(reinterpret_cast<const typename B4<T>::type*>(x) + q, xo);
 #pragma unroll
-        for (int j = 0; j < NC; ++j) s[j] -= ell_row<T>(off, N, p, k, c + j, xo);
+        for (int j = 0; j < NC; ++j) s[j] -= row_dot<T>(o[k][j], xo);
     }
-    dinv_row<T, RT>(dinv, p, c, s, xr);
+    dinv_row<T, RT>(d, s, xr);
     row_store<T, RT>(x, p, c, xr);
 }
 
@@ -557,22 +588,23 @@ __global__ void __launch_bounds__(128) k_imp_gs(const Ell e, const int N, const 
 // first colour of the forward sweep, x_p = D_p^-1 v_p, over its n0 rows.
 template <class T, int RT>
 __global__ void __launch_bounds__(128) k_imp_scale_gs(const Ell e, const int n_rows, const T* __restrict__ dinv,
-                                                      const int n0, const T* __restrict__ w,
-                                                      const double* __restrict__ scale, T* __restrict__ vbase,
-                                                      const int* __restrict__ vk, T* __restrict__ x,
-                                                      const int* __restrict__ stop, const int* __restrict__ case_done) {
+                                                      const int n0, const T* w, const double* scale, T* vbase,
+                                                      const int* vk, T* x, const int* stop,
+                                                      const int* __restrict__ case_done) {
     constexpr int NC = 4 / RT;
-    if (*stop) return;
     const int t = blockIdx.x * blockDim.x + threadIdx.x, p = t / RT, c = NC * (t % RT);
-    if (p >= n_rows) return;
-    const T sc = (T)scale[0];
+    Row<T> d[NC];
+    if (p < n0) diag_rows<T, RT>(dinv, p, c, d);
+    pdl_wait();
+    if (ldw(stop) || p >= n_rows) return;
+    const T sc = (T)ldw(scale);
     T s[NC], xr[NC];
     row_load<T, RT>(w, p, c, s);
 #pragma unroll
     for (int k = 0; k < NC; ++k) s[k] *= sc;
-    row_store<T, RT>(vbase + (long long)*vk * (4 * (long long)n_rows), p, c, s);
+    row_store<T, RT>(vbase + (long long)ldw(vk) * (4 * (long long)n_rows), p, c, s);
     if (p >= n0) return;
-    dinv_row<T, RT>(dinv, p, c, s, xr);
+    dinv_row<T, RT>(d, s, xr);
     if (held(e.case_row, case_done, p)) {
 #pragma unroll
         for (int k = 0; k < NC; ++k) xr[k] = T(0);
@@ -673,10 +705,9 @@ __device__ __forceinline__ Part<T> warp_sums(const T* acc, const int lane) {
 struct GivensCol {
     double col[GM_M + 1], cs[GM_M], sn[GM_M];
 };
-__device__ __forceinline__ void givens_column(GmresCtl* c, const double* __restrict__ h1,
-                                              const double* __restrict__ h2, GivensCol& g) {
+__device__ __forceinline__ void givens_column(GmresCtl* c, const double* h1, const double* h2, GivensCol& g) {
     const int lane = threadIdx.x, j = c->k;
-    for (int t = lane; t <= j; t += 32) g.col[t] = h1[t] + h2[t];
+    for (int t = lane; t <= j; t += 32) g.col[t] = ldw(&h1[t]) + ldw(&h2[t]);
     for (int t = lane; t < j; t += 32) {
         g.cs[t] = c->cs[t];
         g.sn[t] = c->sn[t];
@@ -694,7 +725,7 @@ __device__ __forceinline__ void givens_column(GmresCtl* c, const double* __restr
     __syncwarp();
     for (int t = lane; t <= j; t += 32) c->H[t + (GM_M + 1) * j] = g.col[t];
 }
-__device__ __forceinline__ void givens_finish(GmresCtl* c, const double ww, double* __restrict__ scale) {
+__device__ __forceinline__ void givens_finish(GmresCtl* c, const double ww, double* scale) {
     const int j = c->k;
     double* col = c->H + (GM_M + 1) * j;
     const double hn = sqrt(fmax(ww, 0.0));
@@ -732,7 +763,7 @@ static_assert((GM_M + 2) % DOT_U == 0, "whole groups");
 // counts itself.
 template <class T, int NT, bool ONE>
 __device__ __forceinline__ bool grid_sums(const T* acc, const int nout, const int blk, const int nblk,
-                                          double* __restrict__ part, unsigned* __restrict__ counter, double& total) {
+                                          double* part, unsigned* counter, double& total) {
     const bool adds = blk >= 0;
     constexpr int NW = NT / 32;
     __shared__ double sh[NW][32];
@@ -797,23 +828,39 @@ __device__ __forceinline__ bool grid_sums(const T* acc, const int nout, const in
 // column the step completes, with h1 and hin = h2; scale: 1/||w||
 template <class T, int MODE>
 __global__ void __launch_bounds__(DOT_THREADS, MODE == 1 ? 1 : 2)
-    k_imp_dots(const int n, int nv, const int* __restrict__ nvk, const T* __restrict__ V, T* w,
-               const double* __restrict__ hin, double* __restrict__ part, unsigned* __restrict__ counter,
-               double* __restrict__ out, const int* stop, GmresCtl* givens, const double* __restrict__ h1,
-               double* __restrict__ scale) {
+    k_imp_dots(const int n, int nv, const int* nvk, const T* V, T* w, const double* hin, double* part,
+               unsigned* counter, double* out, const int* stop, GmresCtl* givens, const double* h1, double* scale) {
     __shared__ T hs[GM_M + 2];
     __shared__ GivensCol gc;
-    if (stop && *stop) {
+    // the basis is complete before the predecessor of this kernel started, as is
+    // *nvk: the first chunk's vectors are read ahead of the wait
+    using VT = typename Vec16<T>::type;
+    const int nc = n / Vec16<T>::W;
+    const VT* Vv = reinterpret_cast<const VT*>(V);
+    VT* wv = reinterpret_cast<VT*>(w);
+    // block 0 of an Arnoldi step's MODE 2 sees to the column, the others sum
+    const int first = MODE == 2 && givens ? 1 : 0, blk = (int)blockIdx.x - first, nblk = (int)gridDim.x - first;
+    const bool adds = blk >= 0;
+    if (nvk) nv = ldw(nvk) + 1;  // v_0 .. v_k of the current Arnoldi step
+    constexpr int NV = MODE == 1 ? GM_M + 2 : 2 * DOT_U;  // vectors held in registers
+    VT vv[NV];
+    auto basis = [&](const int i) {
+#pragma unroll
+        for (int j0 = 0; j0 < NV; j0 += DOT_U)
+            if (j0 < nv)
+#pragma unroll
+                for (int j = j0; j < j0 + DOT_U; ++j) vv[j] = j < nv ? ldw(&Vv[(size_t)j * nc + i]) : VT();
+    };
+    const int i0 = blk * blockDim.x + threadIdx.x;
+    if (adds && i0 < nc) basis(i0);
+    pdl_wait();
+    if (stop && ldw(stop)) {
         // an Arnoldi step launched after the cycle's end
         if (MODE == 2 && givens && givens->graph && blockIdx.x == 0 && threadIdx.x == 0)
             cudaGraphSetConditional(givens->hin, 0);
         return;
     }
-    if (nvk) nv = *nvk + 1;  // v_0 .. v_k of the current Arnoldi step
     const int nout = MODE == 2 ? 1 : nv;
-    // block 0 of an Arnoldi step's MODE 2 sees to the column, the others sum
-    const int first = MODE == 2 && givens ? 1 : 0, blk = (int)blockIdx.x - first, nblk = (int)gridDim.x - first;
-    const bool adds = blk >= 0;
     T acc[GM_M + 2];
 #pragma unroll
     for (int j = 0; j < GM_M + 2; ++j) acc[j] = 0;
@@ -823,51 +870,39 @@ __global__ void __launch_bounds__(DOT_THREADS, MODE == 1 ? 1 : 2)
             __threadfence();  // the column is visible before the block is counted
         }
     } else {
-        if (threadIdx.x < GM_M + 2) hs[threadIdx.x] = (int)threadIdx.x < nv ? (T)hin[threadIdx.x] : T(0);
+        if (threadIdx.x < GM_M + 2) hs[threadIdx.x] = (int)threadIdx.x < nv ? (T)ldw(&hin[threadIdx.x]) : T(0);
         __syncthreads();
         // per-thread partial sums in T over 16-byte chunks of the vectors (a few
-        // chunks each; n is 4 * cells, so whole chunks)
-        using VT = typename Vec16<T>::type;
-        const int nc = n / Vec16<T>::W;
-        const VT* __restrict__ Vv = reinterpret_cast<const VT*>(V);
-        VT* wv = reinterpret_cast<VT*>(w);
-        for (int i = blk * blockDim.x + threadIdx.x; i < nc; i += nblk * blockDim.x) {
-            VT wi = wv[i];
-            if (MODE == 1) {
-                // the basis chunks stay in registers for the second product
-                // (one block per SM; the loads of a chunk are all in flight at
-                // once)
-                VT vv[GM_M + 1];
+        // chunks each; n is 4 * cells, so whole chunks); MODE 1 keeps a chunk of
+        // every vector in registers for the second product (one block per SM)
+        for (int i = i0; i < nc; i += nblk * blockDim.x) {
+            VT wi = ldw(&wv[i]);
+            if (i != i0) basis(i);
 #pragma unroll
-                for (int j0 = 0; j0 <= GM_M; j0 += DOT_U)
-                    if (j0 < nv)
+            for (int j0 = 0; j0 < NV; j0 += DOT_U)
+                if (j0 < nv)
 #pragma unroll
-                        for (int j = j0; j < j0 + DOT_U && j <= GM_M; ++j)
-                            vv[j] = j < nv ? Vv[(size_t)j * nc + i] : VT();
+                    for (int j = j0; j < j0 + DOT_U; ++j) vsub(wi, hs[j], vv[j]);
+            if (MODE == 2) {
 #pragma unroll
-                for (int j0 = 0; j0 <= GM_M; j0 += DOT_U)
-                    if (j0 < nv)
-#pragma unroll
-                        for (int j = j0; j < j0 + DOT_U && j <= GM_M; ++j) vsub(wi, hs[j], vv[j]);
-                wv[i] = wi;
-#pragma unroll
-                for (int j0 = 0; j0 <= GM_M; j0 += DOT_U)
-                    if (j0 < nv)
-#pragma unroll
-                        for (int j = j0; j < j0 + DOT_U && j <= GM_M; ++j) acc[j] += vdot(vv[j], wi);
-            } else {
-#pragma unroll
-                for (int j0 = 0; j0 <= GM_M; j0 += DOT_U)
+                for (int j0 = NV; j0 < GM_M + 2; j0 += DOT_U)
                     if (j0 < nv) {
-                        VT vv[DOT_U];
+                        VT u[DOT_U];
 #pragma unroll
-                        for (int u = 0; u < DOT_U; ++u)
-                            vv[u] = j0 + u < nv ? Vv[(size_t)(j0 + u) * nc + i] : VT();
+                        for (int j = 0; j < DOT_U; ++j)
+                            u[j] = j0 + j < nv ? ldw(&Vv[(size_t)(j0 + j) * nc + i]) : VT();
 #pragma unroll
-                        for (int u = 0; u < DOT_U; ++u) vsub(wi, hs[j0 + u], vv[u]);
+                        for (int j = 0; j < DOT_U; ++j) vsub(wi, hs[j0 + j], u[j]);
                     }
                 if (nv > 0) wv[i] = wi;
                 acc[0] += vdot(wi, wi);
+            } else {
+                wv[i] = wi;
+#pragma unroll
+                for (int j0 = 0; j0 < NV; j0 += DOT_U)
+                    if (j0 < nv)
+#pragma unroll
+                        for (int j = j0; j < j0 + DOT_U; ++j) acc[j] += vdot(vv[j], wi);
             }
         }
     }
@@ -883,23 +918,34 @@ __global__ void __launch_bounds__(DOT_THREADS, MODE == 1 ? 1 : 2)
 // pass over w less per Arnoldi step.
 template <class T, int RT>
 __global__ void __launch_bounds__(DOT_THREADS, 2)
-    k_imp_spmv_dots(const int n_rows, const Ell e, const T* __restrict__ dblk, const T* __restrict__ off,
-                    const T* __restrict__ x, T* __restrict__ w, const int* __restrict__ vk, const T* __restrict__ V,
-                    double* __restrict__ part, unsigned* __restrict__ counter, double* __restrict__ out,
-                    const int* __restrict__ stop, const int* __restrict__ case_done) {
+    k_imp_spmv_dots(const int n_rows, const Ell e, const T* __restrict__ dblk, const T* __restrict__ off, const T* x,
+                    T* w, const int* vk, const T* V, double* part, unsigned* counter, double* out, const int* stop,
+                    const int* __restrict__ case_done) {
     constexpr int NC = 4 / RT;
-    if (*stop) return;
-    const int nv = *vk + 1;
+    const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    int4 col = make_int4(-1, -1, -1, -1);
+    Row<T> d[NC];
+    if (t0 < RT * (long long)n_rows) {
+        const int p = (int)(t0 / RT), c = NC * (int)(t0 % RT);
+        col = __ldg(&e.col[p]);
+        diag_rows<T, RT>(dblk, p, c, d);
+    }
+    pdl_wait();
+    if (ldw(stop)) return;
+    const int nv = ldw(vk) + 1;
     T acc[GM_M + 2];
 #pragma unroll
     for (int j = 0; j < GM_M + 2; ++j) acc[j] = 0;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < RT * (long long)n_rows;
-         t += (long long)gridDim.x * blockDim.x) {
+    for (long long t = t0; t < RT * (long long)n_rows; t += (long long)gridDim.x * blockDim.x) {
         const int p = (int)(t / RT), c = NC * (int)(t % RT);
+        if (t != t0) {
+            col = __ldg(&e.col[p]);
+            diag_rows<T, RT>(dblk, p, c, d);
+        }
         T y[NC];
 #pragma unroll
         for (int r = 0; r < NC; ++r) y[r] = T(0);
-        if (!held(e.case_row, case_done, p)) spmv_row<T, RT>(n_rows, e, dblk, off, x, p, c, y);
+        if (!held(e.case_row, case_done, p)) spmv_row<T, RT>(n_rows, col, d, off, x, p, c, y);
         row_store<T, RT>(w, p, c, y);
 #pragma unroll
         for (int j0 = 0; j0 <= GM_M; j0 += DOT_U)
@@ -1289,8 +1335,8 @@ struct Ops {
     T* vec(int j) const { return (T*)e->V + (size_t)j * e->n4; }
     int* stop() const { return &e->ctl->stop; }
     void spmv(const T* x, T* y, const int* st) const {
-        dev::k_imp_spmv<T><<<nb_(e->N, 256), 256, 0, s>>>(e->N, e->ell(), (const T*)e->dblk, (const T*)e->off, x, y,
-                                                          st, a.case_done);
+        launch_pdl(dev::k_imp_spmv<T>, nb_(e->N, 256), 256, 0, s, e->N, e->ell(), (const T*)e->dblk, (const T*)e->off, x,
+                   y, st, a.case_done);
     }
     // t = b in row order
     void gather_b(const double* b, T* t) const {
@@ -1313,25 +1359,21 @@ struct Ops {
             const int c0 = e->color_ptr[c], cn = e->color_ptr[c + 1] - c0;
             if (cn == 0) continue;
             if (four(cn))
-                dev::k_imp_gs<T, 4><<<nb_(4LL * cn, 128), 128, 0, s>>>(e->ell(), e->N, (const T*)e->dinv,
-                                                                       (const T*)e->off, c0, cn, r, rk,
-                                                                       (long long)e->n4, x, st, a.case_done, k < C);
+                launch_pdl(dev::k_imp_gs<T, 4>, nb_(4LL * cn, 128), 128, 0, s, e->ell(), e->N, (const T*)e->dinv,
+                           (const T*)e->off, c0, cn, r, rk, (long long)e->n4, x, st, a.case_done, k < C);
             else
-                dev::k_imp_gs<T, 1><<<nb_(cn, 128), 128, 0, s>>>(e->ell(), e->N, (const T*)e->dinv, (const T*)e->off,
-                                                                 c0, cn, r, rk, (long long)e->n4, x, st, a.case_done,
-                                                                 k < C);
+                launch_pdl(dev::k_imp_gs<T, 1>, nb_(cn, 128), 128, 0, s, e->ell(), e->N, (const T*)e->dinv,
+                           (const T*)e->off, c0, cn, r, rk, (long long)e->n4, x, st, a.case_done, k < C);
         }
     }
     // v_k = w * scale, x = P^-1 v_k (the first colour with the scaling)
     void scale_precond(const T* w, const double* sc, T* V, const int* k, T* x, const int* st) const {
         if (four(e->N))
-            dev::k_imp_scale_gs<T, 4><<<nb_(e->n4, 128), 128, 0, s>>>(e->ell(), e->N, (const T*)e->dinv,
-                                                                      e->color_ptr[1], w, sc, V, k, x, st,
-                                                                      a.case_done);
+            launch_pdl(dev::k_imp_scale_gs<T, 4>, nb_(e->n4, 128), 128, 0, s, e->ell(), e->N, (const T*)e->dinv,
+                       e->color_ptr[1], w, sc, V, k, x, st, a.case_done);
         else
-            dev::k_imp_scale_gs<T, 1><<<nb_(e->N, 128), 128, 0, s>>>(e->ell(), e->N, (const T*)e->dinv,
-                                                                     e->color_ptr[1], w, sc, V, k, x, st,
-                                                                     a.case_done);
+            launch_pdl(dev::k_imp_scale_gs<T, 1>, nb_(e->N, 128), 128, 0, s, e->ell(), e->N, (const T*)e->dinv,
+                       e->color_ptr[1], w, sc, V, k, x, st, a.case_done);
         precond(V, k, x, st, 1);
     }
     // MODE 1: w -= V hin, out = V^T w; 2: w -= V hin, out = w.w
@@ -1339,19 +1381,17 @@ struct Ops {
     void dots(int nv, const int* nvk, const T* V, T* w, const double* hin, double* out, const int* st) const {
         // MODE 1 holds one block per SM
         const int g = MODE == 1 ? e->nbd1 : e->nbd;
-        dev::k_imp_dots<T, MODE><<<g, dev::DOT_THREADS, 0, s>>>(e->n4, nv, nvk, V, w, hin, e->part, e->counter, out,
-                                                              st, nullptr, nullptr, nullptr);
+        launch_pdl(dev::k_imp_dots<T, MODE>, g, dev::DOT_THREADS, 0, s, e->n4, nv, nvk, V, w, hin, e->part, e->counter,
+                   out, st, nullptr, nullptr, nullptr);
     }
     // w = M x, out = V^T w
     void spmv_dots(const T* x, T* w, const int* k, const T* V, double* out, const int* st) const {
         if (four(e->N))
-            dev::k_imp_spmv_dots<T, 4><<<e->nbd, dev::DOT_THREADS, 0, s>>>(
-                e->N, e->ell(), (const T*)e->dblk, (const T*)e->off, x, w, k, V, e->part, e->counter, out, st,
-                a.case_done);
+            launch_pdl(dev::k_imp_spmv_dots<T, 4>, e->nbd, dev::DOT_THREADS, 0, s, e->N, e->ell(), (const T*)e->dblk,
+                       (const T*)e->off, x, w, k, V, e->part, e->counter, out, st, a.case_done);
         else
-            dev::k_imp_spmv_dots<T, 1><<<e->nbd, dev::DOT_THREADS, 0, s>>>(
-                e->N, e->ell(), (const T*)e->dblk, (const T*)e->off, x, w, k, V, e->part, e->counter, out, st,
-                a.case_done);
+            launch_pdl(dev::k_imp_spmv_dots<T, 1>, e->nbd, dev::DOT_THREADS, 0, s, e->N, e->ell(), (const T*)e->dblk,
+                       (const T*)e->off, x, w, k, V, e->part, e->counter, out, st, a.case_done);
     }
     // the end of an Arnoldi step: MODE 2 and column k of the Hessenberg matrix
     // (a block of its own for the earlier rotations, inside the one wave that
@@ -1359,8 +1399,8 @@ struct Ops {
     void finish_step(const int* k, const T* V, T* w, const double* h1, const double* h2, double* ww, double* sc,
                      const int* st) const {
         const int g = std::max(2, std::min(e->nbd + 1, 2 * e->nbd1));
-        dev::k_imp_dots<T, 2><<<g, dev::DOT_THREADS, 0, s>>>(e->n4, 0, k, V, w, h2, e->part, e->counter, ww, st,
-                                                           e->ctl, h1, sc);
+        launch_pdl(dev::k_imp_dots<T, 2>, g, dev::DOT_THREADS, 0, s, e->n4, 0, k, V, w, h2, e->part, e->counter, ww, st,
+                   e->ctl, h1, sc);
     }
     // Arnoldi step k: v_k = w * scale, z = P^-1 v_k, w = M z, CGS2 against
     // v_0..v_k in three passes over the basis (h1 = V^T w; w -= V h1 and
