@@ -525,98 +525,173 @@ __device__ __forceinline__ void dinv_row(const Row<T>* d, const T* s, T* x) {
     for (int r = 0; r < 4 / RT; ++r) x[r] = row_dot<T>(d[r], sv);
 }
 
-// One colour (rows c0 .. c0+n-1) of a block Gauss-Seidel sweep:
-// x_p = D_p^-1 (r_p - sum O x_q).  r = rbase + (*rk) * stride when rk is
-// given (the current Krylov vector).  In the forward sweep only rows of
-// lower colours (q < c0) are read: the higher colours have no value yet
-// (zero start).
+// One row of a block Gauss-Seidel sweep: x_p = D_p^-1 (r_p - sum O x_q) over
+// the slots left in col; its blocks first (`blocks`), the arithmetic after.
 template <class T, int RT>
-__global__ void __launch_bounds__(128) k_imp_gs(const Ell e, const int N, const T* __restrict__ dinv,
-                                                const T* __restrict__ off, const int c0, const int n, const T* rbase,
-                                                const int* rk, const long long stride, T* x, const int* stop,
-                                                const int* __restrict__ case_done, const bool fwd) {
-    constexpr int NC = 4 / RT;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool in = t < n * RT;
-    const int p = c0 + t / RT, c = NC * (t % RT);
-    int4 col = make_int4(-1, -1, -1, -1);
+struct GsRow {
+    static constexpr int NC = 4 / RT;
+    int p, c;
+    int4 col;
     Row<T> d[NC], o[4][NC];
-    auto blocks = [&]() {
+    // `top`: slots of rows from there on are left out (the forward sweep reads
+    // lower colours only: the higher ones have no value yet)
+    __device__ __forceinline__ void at(const Ell& e, const int row, const int comp, const int top) {
+        p = row;
+        c = comp;
+        col = __ldg(&e.col[p]);
+        if (col.x >= top) col.x = -1;
+        if (col.y >= top) col.y = -1;
+        if (col.z >= top) col.z = -1;
+        if (col.w >= top) col.w = -1;
+    }
+    __device__ __forceinline__ void blocks(const T* __restrict__ dinv, const T* __restrict__ off, const int N) {
         diag_rows<T, RT>(dinv, p, c, d);
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             if (pick(col, k) >= 0)
 #pragma unroll
                 for (int j = 0; j < NC; ++j) o[k][j] = ell_row<T>(off, N, p, k, c + j);
-    };
-    if (in) {
-        col = __ldg(&e.col[p]);
-        if (fwd) {
-            if (col.x >= c0) col.x = -1;
-            if (col.y >= c0) col.y = -1;
-            if (col.z >= c0) col.z = -1;
-            if (col.w >= c0) col.w = -1;
+    }
+    __device__ __forceinline__ void solve(const T* r, T* x, const bool is_held) const {
+        T xr[NC];
+        if (is_held) {
+#pragma unroll
+            for (int k = 0; k < NC; ++k) xr[k] = T(0);
+            row_store<T, RT>(x, p, c, xr);
+            return;
         }
-        if (AHEAD<T, RT>) blocks();
+        T s[NC];
+        row_load<T, RT>(r, p, c, s);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int q = pick(col, k);
+            if (q < 0) continue;
+            T xo[4];
+            ldt(reinterpret_cast<const typename B4<T>::type*>(x) + q, xo);
+#pragma unroll
+            for (int j = 0; j < NC; ++j) s[j] -= row_dot<T>(o[k][j], xo);
+        }
+        dinv_row<T, RT>(d, s, xr);
+        row_store<T, RT>(x, p, c, xr);
+    }
+};
+
+// One colour (rows c0 .. c0+n-1) of the sweep.  r = rbase + (*rk) * stride
+// when rk is given (the current Krylov vector).
+template <class T, int RT>
+__global__ void __launch_bounds__(128) k_imp_gs(const Ell e, const int N, const T* __restrict__ dinv,
+                                                const T* __restrict__ off, const int c0, const int n, const T* rbase,
+                                                const int* rk, const long long stride, T* x, const int* stop,
+                                                const int* __restrict__ case_done, const bool fwd) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool in = t < n * RT;
+    GsRow<T, RT> row;
+    if (in) {
+        row.at(e, c0 + t / RT, (4 / RT) * (t % RT), fwd ? c0 : N);
+        if (AHEAD<T, RT>) row.blocks(dinv, off, N);
     }
     pdl_wait();
     if (!in || (stop && ldw(stop))) return;
-    if (!AHEAD<T, RT>) blocks();
-    T xr[NC];
-    if (held(e.case_row, case_done, p)) {
-#pragma unroll
-        for (int k = 0; k < NC; ++k) xr[k] = T(0);
-        row_store<T, RT>(x, p, c, xr);
-        return;
-    }
-    T s[NC];
-    row_load<T, RT>(rbase + (rk ? (long long)ldw(rk) * stride : 0), p, c, s);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int q = pick(col, k);
-        if (q < 0) continue;
-        T xo[4];
-        ldt(reinterpret_cast<const typename B4<T>::type*>(x) + q, xo);
-#pragma unroll
-        for (int j = 0; j < NC; ++j) s[j] -= row_dot<T>(o[k][j], xo);
-    }
-    dinv_row<T, RT>(d, s, xr);
-    row_store<T, RT>(x, p, c, xr);
+    if (!AHEAD<T, RT>) row.blocks(dinv, off, N);
+    row.solve(rbase + (rk ? (long long)ldw(rk) * stride : 0), x, held(e.case_row, case_done, row.p));
 }
 
-// The start of an Arnoldi step: v_k = w * scale[0] over all rows, and the
-// first colour of the forward sweep, x_p = D_p^-1 v_p, over its n0 rows.
+// The top of the sweep in one block: the last colours of a greedy colouring
+// hold a handful of rows (16k quadrilaterals: 6836, 6848, 2140, 554, 6), and
+// each cost a launch on the way up and another on the way down.  Stage j does
+// n[j] rows: c0[j], c0[j]+1, ... (forward), or list[c0[j]], ... (backward, fwd
+// 0): on the way down only rows with a neighbour of a higher colour change, the
+// others would be formed again unchanged.
+constexpr int GS_TAIL = 6;
+struct TailStages {
+    int m;
+    int c0[GS_TAIL], n[GS_TAIL], fwd[GS_TAIL];
+};
+template <class T>
+__global__ void __launch_bounds__(1024) k_imp_gs_tail(const Ell e, const int N, const T* __restrict__ dinv,
+                                                      const T* __restrict__ off, const TailStages st,
+                                                      const int* __restrict__ list, const T* rbase, const int* rk,
+                                                      const long long stride, T* x, const int* stop,
+                                                      const int* __restrict__ case_done) {
+    pdl_wait();
+    if (stop && ldw(stop)) return;
+    constexpr int RT = 4;
+    const T* r = rbase + (rk ? (long long)ldw(rk) * stride : 0);
+    for (int j = 0; j < st.m; ++j) {
+        for (int t = threadIdx.x; t < RT * st.n[j]; t += blockDim.x) {
+            const int i = st.c0[j] + t / RT, p = st.fwd[j] ? i : __ldg(&list[i]);
+            GsRow<T, RT> row;
+            row.at(e, p, t % RT, st.fwd[j] ? st.c0[j] : N);
+            row.blocks(dinv, off, N);
+            row.solve(r, x, held(e.case_row, case_done, p));
+        }
+        __syncthreads();  // the stage's rows are visible to the block
+    }
+}
+
+// The start of Arnoldi step k: the second Gram-Schmidt update of the vector
+// the previous step left, v_k = (w - sum_j h2_j v_j) * scale[0] over j < k (step
+// 0: v_0 = w * scale[0]), and the first colour of the forward sweep,
+// x_p = D_p^-1 v_p, over its n0 rows.  Basis vectors are read DOT_U at a time,
+// all loads of a group before its arithmetic: one after the other each would
+// wait out its own latency.
+constexpr int DOT_U = 8;
+static_assert((GM_M + 2) % DOT_U == 0, "whole groups");
 template <class T, int RT>
-__global__ void __launch_bounds__(128) k_imp_scale_gs(const Ell e, const int n_rows, const T* __restrict__ dinv,
-                                                      const int n0, const T* w, const double* scale, T* vbase,
-                                                      const int* vk, T* x, const int* stop,
+__global__ void __launch_bounds__(128) k_imp_next_vec(const Ell e, const int n_rows, const T* __restrict__ dinv,
+                                                      const int n0, const T* w, const double* h2, const double* scale,
+                                                      T* vbase, const int* vk, T* x, const int* stop,
                                                       const int* __restrict__ case_done) {
     constexpr int NC = 4 / RT;
+    __shared__ T hs[GM_M + 2];
     const int t = blockIdx.x * blockDim.x + threadIdx.x, p = t / RT, c = NC * (t % RT);
     Row<T> d[NC];
     if (p < n0) diag_rows<T, RT>(dinv, p, c, d);
     pdl_wait();
-    if (ldw(stop) || p >= n_rows) return;
+    if (ldw(stop)) return;
+    const int k = ldw(vk);
+    if (threadIdx.x < GM_M + 2) hs[threadIdx.x] = (int)threadIdx.x < k ? (T)ldw(&h2[threadIdx.x]) : T(0);
+    __syncthreads();
+    if (p >= n_rows) return;
     const T sc = (T)ldw(scale);
     T s[NC], xr[NC];
     row_load<T, RT>(w, p, c, s);
+    for (int j0 = 0; j0 < k; j0 += DOT_U) {
+        T v[DOT_U][NC];
 #pragma unroll
-    for (int k = 0; k < NC; ++k) s[k] *= sc;
-    row_store<T, RT>(vbase + (long long)ldw(vk) * (4 * (long long)n_rows), p, c, s);
+        for (int u = 0; u < DOT_U; ++u) {
+#pragma unroll
+            for (int r = 0; r < NC; ++r) v[u][r] = T(0);
+            if (j0 + u < k) row_load<T, RT>(vbase + (size_t)(j0 + u) * 4 * n_rows, p, c, v[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < DOT_U; ++u)
+#pragma unroll
+            for (int r = 0; r < NC; ++r) s[r] -= hs[j0 + u] * v[u][r];
+    }
+#pragma unroll
+    for (int r = 0; r < NC; ++r) s[r] *= sc;
+    row_store<T, RT>(vbase + (size_t)k * 4 * n_rows, p, c, s);
     if (p >= n0) return;
     dinv_row<T, RT>(d, s, xr);
     if (held(e.case_row, case_done, p)) {
 #pragma unroll
-        for (int k = 0; k < NC; ++k) xr[k] = T(0);
+        for (int r = 0; r < NC; ++r) xr[r] = T(0);
     }
     row_store<T, RT>(x, p, c, xr);
 }
 
-// Dot products against the Krylov basis v_0..v_{nv-1} (v_j = V + j*n) in
-// one pass, with the Gram-Schmidt update fused in:
-//   MODE 1: w -= sum_j hin_j v_j, then out_j = v_j . w   (CGS pass 1 + dots of pass 2)
-//   MODE 2: w -= sum_j hin_j v_j, then out_0 = w . w     (CGS pass 2 + the norm; nv = 0: the norm alone)
-// (the dots of pass 1 are formed with w = M x, k_imp_spmv_dots)
+// Classical Gram-Schmidt twice against the Krylov basis v_0..v_{nv-1}
+// (v_j = V + j*n), in three passes over it and two reductions:
+//   k_imp_spmv_dots   w = M x, h1 = V^T w
+//   k_imp_cgs         w -= V h1, h2 = V^T w and w.w
+//   k_imp_next_vec    w -= V h2, scaled to v_{k+1}, by the next step
+// The norm after the second update comes from Pythagoras, w.w - h2.h2 (the
+// basis is orthonormal and h2 a rounding correction), so the second update
+// needs no reduction of its own.  (Were it inaccurate, as it is at a
+// breakdown, v_{k+1} would not have unit length, but the Arnoldi relation
+// would still hold: the vector is divided by the same number that enters the
+// matrix.)
 // The per-thread sums of all outputs are reduced across a warp together: a
 // butterfly that halves the outputs a lane holds at every step takes 31 (16
 // for up to 16 outputs) additions of a warp instead of 5 per output -- in
@@ -625,11 +700,7 @@ __global__ void __launch_bounds__(128) k_imp_scale_gs(const Ell e, const int n_r
 // two-sum, 48 bits) on the FP32 lanes; double takes over after it.  Each block
 // writes its partial sums; the last block to finish adds them in a fixed
 // pattern (a warp per group of blocks, then over the warps), so the result is
-// deterministic, and re-arms the counter.  In MODE 2 of an Arnoldi step one more block applies the earlier
-// Givens rotations to the new column meanwhile, and the last block adds the
-// new rotation.  One Arnoldi step's product, three passes, column and scaling
-// at 16k rows in FP64: 91 -> 42 us in 4 launches instead of 6; at 131k rows in
-// FP32: 68 -> 41 us.
+// deterministic, and re-arms the counter.
 // 16-byte chunks of a vector in T, their dot product and w -= h v
 template <class T> struct Vec16;
 template <> struct Vec16<float> { using type = float4; static constexpr int W = 4; };
@@ -697,65 +768,64 @@ __device__ __forceinline__ Part<T> warp_sums(const T* acc, const int lane) {
 }
 
 // Arnoldi step j = c->k, classical Gram-Schmidt twice: h1 (first pass) and
-// h2 (second pass) sum to column j.  givens_column applies the rotations of
-// the earlier steps to it (one warp, staged in shared memory so the chain runs
-// on shared memory, not on dependent global loads) while the second pass's
-// update is still running; givens_finish adds the subdiagonal entry sqrt(ww),
-// its rotation and the residual estimate.
+// h2 (second pass) sum to column j, ww is the squared norm after the second.
+// One warp, the earlier rotations staged in shared memory ahead of time
+// (givens_stage), so the chain runs on shared memory, not on dependent global
+// loads; then the new subdiagonal entry, its rotation and the residual
+// estimate.
 struct GivensCol {
-    double col[GM_M + 1], cs[GM_M], sn[GM_M];
+    double col[GM_M + 2], cs[GM_M], sn[GM_M];
 };
-__device__ __forceinline__ void givens_column(GmresCtl* c, const double* h1, const double* h2, GivensCol& g) {
-    const int lane = threadIdx.x, j = c->k;
-    for (int t = lane; t <= j; t += 32) g.col[t] = ldw(&h1[t]) + ldw(&h2[t]);
-    for (int t = lane; t < j; t += 32) {
-        g.cs[t] = c->cs[t];
-        g.sn[t] = c->sn[t];
+__device__ __forceinline__ void givens_stage(const GmresCtl* c, const double* h1, const int j, GivensCol& g) {
+    const int t = threadIdx.x;
+    if (t <= j) g.col[t] = ldw(&h1[t]);
+    if (t < j) {
+        g.cs[t] = ldw(&c->cs[t]);
+        g.sn[t] = ldw(&c->sn[t]);
     }
+}
+__device__ __forceinline__ void givens(GmresCtl* c, const double h2, const double sq, GivensCol& g, double* scale) {
+    using namespace fp64;
+    const int lane = threadIdx.x, j = c->k;
+    // sq: w.w after the first update in lane j + 1; h2 in lanes 0..j
+    if (lane <= j) g.col[lane] += h2;
+    double hh = lane <= j ? h2 * h2 : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) hh += __shfl_xor_sync(0xffffffffu, hh, o);
+    const double ww = __shfl_sync(0xffffffffu, sq, j + 1) - hh;
     __syncwarp();
     if (lane == 0) {
+        const double gj = c->g[j], tol = c->tol;
+        const int iters = c->iters + 1, max_iters = c->max_iters;
         double a = g.col[0];
         for (int i = 0; i < j; ++i) {
             const double b = g.col[i + 1];
             g.col[i] = g.cs[i] * a + g.sn[i] * b;
             a = -g.sn[i] * a + g.cs[i] * b;
         }
-        g.col[j] = a;
+        const double hn = root(fmax(ww, 0.0));
+        c->hnext = hn;
+        scale[0] = hn > 0 ? div(1.0, hn) : 0.0;
+        const double b = hn, r = root(a * a + b * b);
+        const Den ir = den(r);
+        const double cj = r > 0 ? quot(a, ir) : 1.0, sj = r > 0 ? quot(b, ir) : 0.0;
+        c->cs[j] = cj;
+        c->sn[j] = sj;
+        g.col[j] = r;
+        g.col[j + 1] = 0;
+        const double res = fabs(sj * gj);
+        c->g[j + 1] = -sj * gj;
+        c->g[j] = cj * gj;
+        c->res = res;
+        c->k = j + 1;
+        c->iters = iters;
+        const int st = (res <= tol || j + 1 == GM_M || hn == 0 || iters >= max_iters) ? 1 : 0;
+        c->stop = st;
+        if (c->graph) cudaGraphSetConditional(c->hin, st ? 0 : 1);
     }
     __syncwarp();
-    for (int t = lane; t <= j; t += 32) c->H[t + (GM_M + 1) * j] = g.col[t];
+    for (int t = lane; t <= j + 1; t += 32) c->H[t + (GM_M + 1) * j] = g.col[t];
 }
-__device__ __forceinline__ void givens_finish(GmresCtl* c, const double ww, double* scale) {
-    const int j = c->k;
-    double* col = c->H + (GM_M + 1) * j;
-    const double hn = sqrt(fmax(ww, 0.0));
-    c->hnext = hn;
-    scale[0] = hn > 0 ? 1.0 / hn : 0.0;
-    const double a = __ldcg(&col[j]), b = hn;
-    const double r = sqrt(a * a + b * b);
-    const double cj = r > 0 ? a / r : 1.0, sj = r > 0 ? b / r : 0.0;
-    c->cs[j] = cj;
-    c->sn[j] = sj;
-    col[j] = r;
-    col[j + 1] = 0;
-    const double g = c->g[j];
-    const double res = fabs(sj * g);
-    const int iters = c->iters + 1;
-    c->g[j + 1] = -sj * g;
-    c->g[j] = cj * g;
-    c->res = res;
-    c->k = j + 1;
-    c->iters = iters;
-    const int st = (res <= c->tol || j + 1 == GM_M || hn == 0 || iters >= c->max_iters) ? 1 : 0;
-    c->stop = st;
-    if (c->graph) cudaGraphSetConditional(c->hin, st ? 0 : 1);
-}
-
-// Basis vectors are read DOT_U at a time, all loads of a group before its
-// arithmetic: one after the other each load would wait out its own latency
-// (3 TB/s at 32 MB of basis).
-constexpr int DOT_U = 8;
-static_assert((GM_M + 2) % DOT_U == 0, "whole groups");
 
 // The block's and, in the last block to finish, the whole sum of the threads'
 // acc[0..nout-1] over blocks 0..nblk-1 of NT threads; true in the last block's
@@ -824,93 +894,86 @@ __device__ __forceinline__ bool grid_sums(const T* acc, const int nout, const in
     return true;
 }
 
-// givens (MODE 2 of an Arnoldi step, else null): the control block whose
-// column the step completes, with h1 and hin = h2; scale: 1/||w||
-template <class T, int MODE>
-__global__ void __launch_bounds__(DOT_THREADS, MODE == 1 ? 1 : 2)
-    k_imp_dots(const int n, int nv, const int* nvk, const T* V, T* w, const double* hin, double* part,
-               unsigned* counter, double* out, const int* stop, GmresCtl* givens, const double* h1, double* scale) {
+// w -= sum_j h1_j v_j, then h2_j = v_j . w and w.w, and in the last block the
+// step's column.  A chunk of every vector stays in registers for the second
+// product (one block per SM); the first chunk's are read ahead of the wait (the
+// basis is complete before this kernel's predecessor started, as is *vk).
+template <class T>
+__global__ void __launch_bounds__(DOT_THREADS, 1) k_imp_cgs(const int n, const T* V, T* w, const double* h1,
+                                                            double* part, unsigned* counter, double* h2, GmresCtl* c,
+                                                            double* scale) {
     __shared__ T hs[GM_M + 2];
     __shared__ GivensCol gc;
-    // the basis is complete before the predecessor of this kernel started, as is
-    // *nvk: the first chunk's vectors are read ahead of the wait
     using VT = typename Vec16<T>::type;
-    const int nc = n / Vec16<T>::W;
+    const int nc = n / Vec16<T>::W, nv = ldw(&c->k) + 1;
     const VT* Vv = reinterpret_cast<const VT*>(V);
     VT* wv = reinterpret_cast<VT*>(w);
-    // block 0 of an Arnoldi step's MODE 2 sees to the column, the others sum
-    const int first = MODE == 2 && givens ? 1 : 0, blk = (int)blockIdx.x - first, nblk = (int)gridDim.x - first;
-    const bool adds = blk >= 0;
-    if (nvk) nv = ldw(nvk) + 1;  // v_0 .. v_k of the current Arnoldi step
-    constexpr int NV = MODE == 1 ? GM_M + 2 : 2 * DOT_U;  // vectors held in registers
-    VT vv[NV];
+    VT vv[GM_M + 1];
     auto basis = [&](const int i) {
 #pragma unroll
-        for (int j0 = 0; j0 < NV; j0 += DOT_U)
+        for (int j0 = 0; j0 <= GM_M; j0 += DOT_U)
             if (j0 < nv)
 #pragma unroll
-                for (int j = j0; j < j0 + DOT_U; ++j) vv[j] = j < nv ? ldw(&Vv[(size_t)j * nc + i]) : VT();
+                for (int j = j0; j < j0 + DOT_U && j <= GM_M; ++j)
+                    vv[j] = j < nv ? ldw(&Vv[(size_t)j * nc + i]) : VT();
     };
-    const int i0 = blk * blockDim.x + threadIdx.x;
-    if (adds && i0 < nc) basis(i0);
+    const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i0 < nc) basis(i0);
     pdl_wait();
-    if (stop && ldw(stop)) {
-        // an Arnoldi step launched after the cycle's end
-        if (MODE == 2 && givens && givens->graph && blockIdx.x == 0 && threadIdx.x == 0)
-            cudaGraphSetConditional(givens->hin, 0);
+    if (ldw(&c->stop)) {  // a step launched after the cycle's end
+        if (c->graph && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(c->hin, 0);
         return;
     }
-    const int nout = MODE == 2 ? 1 : nv;
-    T acc[GM_M + 2];
+    if (threadIdx.x < GM_M + 2) hs[threadIdx.x] = (int)threadIdx.x < nv ? (T)ldw(&h1[threadIdx.x]) : T(0);
+    if (threadIdx.x < 32) givens_stage(c, h1, nv - 1, gc);
+    __syncthreads();
+    // per-thread partial sums in T over 16-byte chunks of the vectors (a few
+    // chunks each; n is 4 * cells, so whole chunks)
+    T acc[GM_M + 2], sq = 0;
 #pragma unroll
     for (int j = 0; j < GM_M + 2; ++j) acc[j] = 0;
-    if (!adds) {
-        if (threadIdx.x < 32) {
-            givens_column(givens, h1, hin, gc);
-            __threadfence();  // the column is visible before the block is counted
-        }
-    } else {
-        if (threadIdx.x < GM_M + 2) hs[threadIdx.x] = (int)threadIdx.x < nv ? (T)ldw(&hin[threadIdx.x]) : T(0);
-        __syncthreads();
-        // per-thread partial sums in T over 16-byte chunks of the vectors (a few
-        // chunks each; n is 4 * cells, so whole chunks); MODE 1 keeps a chunk of
-        // every vector in registers for the second product (one block per SM)
-        for (int i = i0; i < nc; i += nblk * blockDim.x) {
-            VT wi = ldw(&wv[i]);
-            if (i != i0) basis(i);
+    for (int i = i0; i < nc; i += gridDim.x * blockDim.x) {
+        VT wi = ldw(&wv[i]);
+        if (i != i0) basis(i);
 #pragma unroll
-            for (int j0 = 0; j0 < NV; j0 += DOT_U)
-                if (j0 < nv)
+        for (int j0 = 0; j0 <= GM_M; j0 += DOT_U)
+            if (j0 < nv)
 #pragma unroll
-                    for (int j = j0; j < j0 + DOT_U; ++j) vsub(wi, hs[j], vv[j]);
-            if (MODE == 2) {
+                for (int j = j0; j < j0 + DOT_U && j <= GM_M; ++j) vsub(wi, hs[j], vv[j]);
+        wv[i] = wi;
+        sq += vdot(wi, wi);
 #pragma unroll
-                for (int j0 = NV; j0 < GM_M + 2; j0 += DOT_U)
-                    if (j0 < nv) {
-                        VT u[DOT_U];
+        for (int j0 = 0; j0 <= GM_M; j0 += DOT_U)
+            if (j0 < nv)
 #pragma unroll
-                        for (int j = 0; j < DOT_U; ++j)
-                            u[j] = j0 + j < nv ? ldw(&Vv[(size_t)(j0 + j) * nc + i]) : VT();
+                for (int j = j0; j < j0 + DOT_U && j <= GM_M; ++j) acc[j] += vdot(vv[j], wi);
+    }
+    // output nv (at most GM_M) is w.w
 #pragma unroll
-                        for (int j = 0; j < DOT_U; ++j) vsub(wi, hs[j0 + j], u[j]);
-                    }
-                if (nv > 0) wv[i] = wi;
-                acc[0] += vdot(wi, wi);
-            } else {
-                wv[i] = wi;
-#pragma unroll
-                for (int j0 = 0; j0 < NV; j0 += DOT_U)
-                    if (j0 < nv)
-#pragma unroll
-                        for (int j = j0; j < j0 + DOT_U; ++j) acc[j] += vdot(vv[j], wi);
-            }
-        }
+    for (int j = 1; j < GM_M + 2; ++j)
+        if (j == nv) acc[j] = sq;
+    double t = 0;
+    const bool mine = grid_sums<T, DOT_THREADS, false>(acc, nv + 1, (int)blockIdx.x, (int)gridDim.x, part, counter, t);
+    if (!__syncthreads_or(mine) || threadIdx.x >= 32) return;
+    if ((int)threadIdx.x < nv) h2[threadIdx.x] = t;
+    givens(c, t, t, gc, scale);
+}
+
+// out = w.w
+template <class T>
+__global__ void __launch_bounds__(DOT_THREADS) k_imp_sq(const int n, const T* w, double* part, unsigned* counter,
+                                                        double* out, const int* stop) {
+    pdl_wait();
+    if (stop && ldw(stop)) return;
+    using VT = typename Vec16<T>::type;
+    const VT* wv = reinterpret_cast<const VT*>(w);
+    T acc[1] = {0};
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n / Vec16<T>::W; i += gridDim.x * blockDim.x) {
+        const VT wi = ldw(&wv[i]);
+        acc[0] += vdot(wi, wi);
     }
     double t;
-    if (grid_sums<T, DOT_THREADS, MODE == 2>(acc, nout, blk, nblk, part, counter, t)) {
-        out[threadIdx.x] = t;
-        if (MODE == 2 && givens) givens_finish(givens, t, scale);
-    }
+    if (grid_sums<T, DOT_THREADS, true>(acc, 1, (int)blockIdx.x, (int)gridDim.x, part, counter, t)) out[0] = t;
 }
 
 // w = M x and out_j = v_j . w, j <= *vk, in one pass over the rows: the
@@ -1167,6 +1230,11 @@ struct ImplicitEngine {
     cudaStream_t s2 = nullptr, s3 = nullptr;      // capture streams of the loop bodies
     const void* cyc_b = nullptr;                  // right-hand side the graphs were captured with
     int nbd = 0, nbd1 = 0;  // blocks of the dot passes (two / one per SM)
+    // the top of the sweep as one launch (k_imp_gs_tail): up from colour tail0,
+    // down to colour tail_down; rows of a backward stage in blist
+    int tail0 = 0, tail_down = 0;
+    dev::TailStages tail{};
+    int* blist = nullptr;
     dev::GmresCtl* ctl = nullptr;
     dev::GmresCtl* h_ctl = nullptr;
     int last_iters = 0;
@@ -1217,6 +1285,54 @@ ImplicitEngine* implicit_create(const StepArgs& a, bool f32, bool graph, const s
                 if (std::abs(eface[4 * (size_t)q + k2]) == f) etr[4 * (size_t)p + k] = 4 * q + k2;
             if (etr[4 * (size_t)p + k] < 0) throw Error(7, "implicit solver: face slots are not symmetric");
         }
+    // the sweep's top: forward stages of the last colours, then backward ones
+    // over the rows with a neighbour of a higher colour, as long as one block
+    // does them faster than the launches they save.  In FP64 one SM's two lanes
+    // need 1.5 us for 64 rows (with 600 rows in the tail a step at 16k rows
+    // took 12 us longer)
+    const int TAIL_ROWS = e->f32 ? 640 : 64;
+    std::vector<int> blist;
+    auto higher = [&](int c) {
+        std::vector<int> rows;
+        for (int p = e->color_ptr[c]; p < e->color_ptr[c + 1]; ++p)
+            for (int k = 0; k < 4; ++k)
+                if (ecol[4 * (size_t)p + k] >= e->color_ptr[c + 1]) {
+                    rows.push_back(p);
+                    break;
+                }
+        return rows;
+    };
+    int budget = TAIL_ROWS, t0 = nc;
+    while (t0 > 1 && nc - t0 < dev::GS_TAIL / 2 && e->color_ptr[t0] - e->color_ptr[t0 - 1] <= budget) {
+        --t0;
+        budget -= e->color_ptr[t0 + 1] - e->color_ptr[t0];
+    }
+    e->tail0 = t0;
+    e->tail_down = nc - 1;
+    if (t0 < nc) {
+        for (int c = t0; c < nc; ++c) {
+            const int k = e->tail.m++;
+            e->tail.c0[k] = e->color_ptr[c];
+            e->tail.n[k] = e->color_ptr[c + 1] - e->color_ptr[c];
+            e->tail.fwd[k] = 1;
+        }
+        for (int c = nc - 2; c >= std::max(t0 - 1, 0) && e->tail.m < dev::GS_TAIL; --c) {
+            const std::vector<int> rows = higher(c);
+            if ((int)rows.size() > budget) break;
+            budget -= (int)rows.size();
+            const int k = e->tail.m++;
+            e->tail.c0[k] = (int)blist.size();
+            e->tail.n[k] = (int)rows.size();
+            e->tail.fwd[k] = 0;
+            blist.insert(blist.end(), rows.begin(), rows.end());
+            e->tail_down = c;
+        }
+        if (e->tail.m < 2) {  // nothing saved
+            e->tail.m = 0;
+            e->tail0 = nc;
+            e->tail_down = nc - 1;
+        }
+    }
     const size_t T = e->ts();
     auto chk = [](cudaError_t r) {
         if (r != cudaSuccess) throw Error(7, std::string("implicit solver: ") + cudaGetErrorString(r));
@@ -1230,6 +1346,8 @@ ImplicitEngine* implicit_create(const StepArgs& a, bool f32, bool graph, const s
     chk(cudaMalloc((void**)&e->ell_col, N1 * sizeof(int4)));
     chk(cudaMalloc((void**)&e->ell_face, N1 * sizeof(int4)));
     chk(cudaMalloc((void**)&e->ell_tr, N1 * sizeof(int4)));
+    chk(cudaMalloc((void**)&e->blist, std::max<size_t>(blist.size(), 1) * sizeof(int)));
+    chk(cudaMemcpyAsync(e->blist, blist.data(), blist.size() * sizeof(int), cudaMemcpyHostToDevice, s));
     chk(cudaMalloc((void**)&e->singular, sizeof(int)));
     chk(cudaMalloc(&e->V, (size_t)(dev::GM_M + 1) * e->n4 * T));
     chk(cudaMalloc(&e->w, (size_t)e->n4 * T));
@@ -1270,7 +1388,7 @@ void implicit_destroy(ImplicitEngine* e) {
     if (e->s2) cudaStreamDestroy(e->s2);
     if (e->s3) cudaStreamDestroy(e->s3);
     for (void* p : {e->jf, e->dblk, e->dinv, e->off, (void*)e->perm, (void*)e->ell_col, (void*)e->ell_face,
-                    (void*)e->ell_tr, (void*)e->case_row, (void*)e->singular, e->V, e->w, e->z, e->t, (void*)e->x,
+                    (void*)e->ell_tr, (void*)e->blist, (void*)e->case_row, (void*)e->singular, e->V, e->w, e->z, e->t, (void*)e->x,
                     (void*)e->part, (void*)e->small, (void*)e->ctl, (void*)e->counter})
         if (p) cudaFree(p);
     if (e->h_ctl) cudaFreeHost(e->h_ctl);
@@ -1352,65 +1470,48 @@ struct Ops {
     // Krylov vector V + k*n when rk is given.  The forward sweep forms every
     // cell (reading lower colours only) from colour `first` on; the backward
     // sweep skips the top colour, whose value it would form again unchanged.
+    // The sweep's top, from colour e->tail0 up and down again, is one launch.
     void precond(const T* r, const int* rk, T* x, const int* st, int first = 0) const {
-        const int C = e->n_colors;
-        for (int k = first; k < 2 * C - 1; ++k) {
-            const int c = k < C ? k : 2 * C - 2 - k;
+        auto colour = [&](int c, bool fwd) {
             const int c0 = e->color_ptr[c], cn = e->color_ptr[c + 1] - c0;
-            if (cn == 0) continue;
+            if (cn == 0) return;
             if (four(cn))
                 launch_pdl(dev::k_imp_gs<T, 4>, nb_(4LL * cn, 128), 128, 0, s, e->ell(), e->N, (const T*)e->dinv,
-                           (const T*)e->off, c0, cn, r, rk, (long long)e->n4, x, st, a.case_done, k < C);
+                           (const T*)e->off, c0, cn, r, rk, (long long)e->n4, x, st, a.case_done, fwd);
             else
                 launch_pdl(dev::k_imp_gs<T, 1>, nb_(cn, 128), 128, 0, s, e->ell(), e->N, (const T*)e->dinv,
-                           (const T*)e->off, c0, cn, r, rk, (long long)e->n4, x, st, a.case_done, k < C);
-        }
+                           (const T*)e->off, c0, cn, r, rk, (long long)e->n4, x, st, a.case_done, fwd);
+        };
+        const int C = e->n_colors, t0 = std::max(e->tail0, first);
+        const bool tail = e->tail.m > 0 && t0 == e->tail0;
+        for (int c = first; c < (tail ? t0 : C); ++c) colour(c, true);
+        if (tail)
+            launch_pdl(dev::k_imp_gs_tail<T>, 1, 1024, 0, s, e->ell(), e->N, (const T*)e->dinv, (const T*)e->off,
+                       e->tail, e->blist, r, rk, (long long)e->n4, x, st, a.case_done);
+        for (int c = (tail ? e->tail_down : C - 1) - 1; c >= 0; --c) colour(c, false);
     }
-    // v_k = w * scale, x = P^-1 v_k (the first colour with the scaling)
-    void scale_precond(const T* w, const double* sc, T* V, const int* k, T* x, const int* st) const {
-        if (four(e->N))
-            launch_pdl(dev::k_imp_scale_gs<T, 4>, nb_(e->n4, 128), 128, 0, s, e->ell(), e->N, (const T*)e->dinv,
-                       e->color_ptr[1], w, sc, V, k, x, st, a.case_done);
-        else
-            launch_pdl(dev::k_imp_scale_gs<T, 1>, nb_(e->N, 128), 128, 0, s, e->ell(), e->N, (const T*)e->dinv,
-                       e->color_ptr[1], w, sc, V, k, x, st, a.case_done);
-        precond(V, k, x, st, 1);
+    // out = w.w
+    void norm2(const T* w, double* out, const int* st) const {
+        launch_pdl(dev::k_imp_sq<T>, e->nbd, dev::DOT_THREADS, 0, s, e->n4, w, e->part, e->counter, out, st);
     }
-    // MODE 1: w -= V hin, out = V^T w; 2: w -= V hin, out = w.w
-    template <int MODE>
-    void dots(int nv, const int* nvk, const T* V, T* w, const double* hin, double* out, const int* st) const {
-        // MODE 1 holds one block per SM
-        const int g = MODE == 1 ? e->nbd1 : e->nbd;
-        launch_pdl(dev::k_imp_dots<T, MODE>, g, dev::DOT_THREADS, 0, s, e->n4, nv, nvk, V, w, hin, e->part, e->counter,
-                   out, st, nullptr, nullptr, nullptr);
-    }
-    // w = M x, out = V^T w
-    void spmv_dots(const T* x, T* w, const int* k, const T* V, double* out, const int* st) const {
-        if (four(e->N))
+    // Arnoldi step k: v_k from the vector the last step left, z = P^-1 v_k,
+    // w = M z, CGS2 against v_0..v_k, column k of the Hessenberg matrix
+    void arnoldi_step(T* V, T* w, T* z, double* h1, double* h2, double* sc, const int* k, const int* st) const {
+        if (four(e->N)) {
+            launch_pdl(dev::k_imp_next_vec<T, 4>, nb_(e->n4, 128), 128, 0, s, e->ell(), e->N, (const T*)e->dinv,
+                       e->color_ptr[1], w, h2, sc, V, k, z, st, a.case_done);
+            precond(V, k, z, st, 1);
             launch_pdl(dev::k_imp_spmv_dots<T, 4>, e->nbd, dev::DOT_THREADS, 0, s, e->N, e->ell(), (const T*)e->dblk,
-                       (const T*)e->off, x, w, k, V, e->part, e->counter, out, st, a.case_done);
-        else
+                       (const T*)e->off, z, w, k, V, e->part, e->counter, h1, st, a.case_done);
+        } else {
+            launch_pdl(dev::k_imp_next_vec<T, 1>, nb_(e->N, 128), 128, 0, s, e->ell(), e->N, (const T*)e->dinv,
+                       e->color_ptr[1], w, h2, sc, V, k, z, st, a.case_done);
+            precond(V, k, z, st, 1);
             launch_pdl(dev::k_imp_spmv_dots<T, 1>, e->nbd, dev::DOT_THREADS, 0, s, e->N, e->ell(), (const T*)e->dblk,
-                       (const T*)e->off, x, w, k, V, e->part, e->counter, out, st, a.case_done);
-    }
-    // the end of an Arnoldi step: MODE 2 and column k of the Hessenberg matrix
-    // (a block of its own for the earlier rotations, inside the one wave that
-    // two blocks per SM make: a 305th block would wait for another to end)
-    void finish_step(const int* k, const T* V, T* w, const double* h1, const double* h2, double* ww, double* sc,
-                     const int* st) const {
-        const int g = std::max(2, std::min(e->nbd + 1, 2 * e->nbd1));
-        launch_pdl(dev::k_imp_dots<T, 2>, g, dev::DOT_THREADS, 0, s, e->n4, 0, k, V, w, h2, e->part, e->counter, ww, st,
-                   e->ctl, h1, sc);
-    }
-    // Arnoldi step k: v_k = w * scale, z = P^-1 v_k, w = M z, CGS2 against
-    // v_0..v_k in three passes over the basis (h1 = V^T w; w -= V h1 and
-    // h2 = V^T w; w -= V h2 and ||w||^2), rotations
-    void arnoldi_step(T* V, T* w, T* z, double* h1, double* h2, double* ww, double* sc, const int* k,
-                      const int* st) const {
-        scale_precond(w, sc, V, k, z, st);
-        spmv_dots(z, w, k, V, h1, st);
-        dots<1>(0, k, V, w, h1, h2, st);
-        finish_step(k, V, w, h1, h2, ww, sc, st);
+                       (const T*)e->off, z, w, k, V, e->part, e->counter, h1, st, a.case_done);
+        }
+        launch_pdl(dev::k_imp_cgs<T>, e->nbd1, dev::DOT_THREADS, 0, s, e->n4, V, w, h1, e->part, e->counter, h2,
+                   e->ctl, sc);
     }
 };
 
@@ -1463,7 +1564,7 @@ cudaGraphExec_t build_gmres_graph(ImplicitEngine* e, const Ops<T>& o0, const dou
     T* w = (T*)e->w;  // the vector that becomes v_0 (scaled by the first Arnoldi step)
     cudaMemsetAsync(e->x, 0, (size_t)n * 8, s);
     o.gather_b(b, w);
-    o.template dots<2>(0, nullptr, nullptr, w, nullptr, ww, nullptr);
+    o.norm2(w, ww, nullptr);
     k_imp_cycle_init<<<1, 1, 0, s>>>(e->ctl, ww, scale, 1, 1e-2, max_iters);
     cudaGraph_t body_out = add_while(s, &hout);
     cudaMemcpyAsync(e->h_ctl, e->ctl, sizeof(GmresCtl), cudaMemcpyDeviceToHost, s);
@@ -1483,12 +1584,12 @@ cudaGraphExec_t build_gmres_graph(ImplicitEngine* e, const Ops<T>& o0, const dou
         k_imp_cast<T><<<nb_(n, 256), 256, 0, s2>>>(n, e->x, (T*)e->t, halt);
         q.spmv((const T*)e->t, (T*)e->z, halt);
         k_imp_resid<T><<<nb_(n, 256), 256, 0, s2>>>(n, b, e->perm, (const T*)e->z, w, halt);
-        q.template dots<2>(0, nullptr, nullptr, w, nullptr, ww, halt);
+        q.norm2(w, ww, halt);
         k_imp_cycle_init<<<1, 1, 0, s2>>>(e->ctl, ww, scale, 0, 1e-2, max_iters);
         chk(cudaStreamEndCapture(s2, &body_out));
         chk(cudaStreamBeginCaptureToGraph(s3, body_in, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
         Ops<T> r(e, o0.a, s3);
-        r.arnoldi_step(r.vec(0), w, (T*)e->z, h1, h2, ww, scale, kptr, stop);
+        r.arnoldi_step(r.vec(0), w, (T*)e->z, h1, h2, scale, kptr, stop);
         chk(cudaStreamEndCapture(s3, &body_in));
     }
     cudaGraphExec_t ex;
@@ -1527,7 +1628,7 @@ int gmres_host_loop(ImplicitEngine* e, const StepArgs& a, const double* b, cudaS
     T* w = (T*)e->w;
     cudaMemsetAsync(e->x, 0, (size_t)n * 8, s);
     o.gather_b(b, w);
-    o.template dots<2>(0, nullptr, nullptr, w, nullptr, ww, nullptr);
+    o.norm2(w, ww, nullptr);
     k_imp_cycle_init<<<1, 1, 0, s>>>(e->ctl, ww, scale, 1, 1e-2, max_iters);
     read_ctl();
     if (!e->h_ctl->stop) {
@@ -1535,7 +1636,7 @@ int gmres_host_loop(ImplicitEngine* e, const StepArgs& a, const double* b, cudaS
             for (;;) {  // Arnoldi steps of the cycle
                 read_ctl();
                 if (e->h_ctl->stop) break;
-                o.arnoldi_step(o.vec(0), w, (T*)e->z, h1, h2, ww, scale, kptr, stop);
+                o.arnoldi_step(o.vec(0), w, (T*)e->z, h1, h2, scale, kptr, stop);
             }
             k_imp_solve_y<<<1, 32, 0, s>>>(e->ctl);
             k_imp_lincomb<T><<<nb_(n, 256), 256, 0, s>>>(n, o.vec(0), e->ctl, (T*)e->t);
@@ -1545,7 +1646,7 @@ int gmres_host_loop(ImplicitEngine* e, const StepArgs& a, const double* b, cudaS
             k_imp_cast<T><<<nb_(n, 256), 256, 0, s>>>(n, e->x, (T*)e->t, halt);
             o.spmv((const T*)e->t, (T*)e->z, halt);
             k_imp_resid<T><<<nb_(n, 256), 256, 0, s>>>(n, b, e->perm, (const T*)e->z, w, halt);
-            o.template dots<2>(0, nullptr, nullptr, w, nullptr, ww, halt);
+            o.norm2(w, ww, halt);
             k_imp_cycle_init<<<1, 1, 0, s>>>(e->ctl, ww, scale, 0, 1e-2, max_iters);
             read_ctl();
             if (e->h_ctl->halt) break;
