@@ -262,10 +262,8 @@ struct afx_solver_s {
     struct AdjointBufs {
         DevBuf v, fbar, gbx, gby, qbar, lw, lt, u, bqbar, g, q, lam[2], ls[2], partials;
         DevBuf lam_obj[2];  // the last implicit adjoint solution of C_L / C_D (initial guess of the next)
-        int dirs = 4;       // input directions per pass of the face kernel
         AdjArgs args(const void* v_dev, void* u_dev) const {
             AdjArgs j;
-            j.dirs_per_pass = dirs;
             j.v = v_dev;
             j.fbar = fbar.p;
             j.gbx = gbx.p;
@@ -298,7 +296,6 @@ struct afx_solver_s {
         if (!adj) {
             const size_t N = a.n_cells, F = a.n_faces, B = std::max(a.n_bnd, 1);
             auto b = std::make_unique<AdjointBufs>();
-            b->dirs = st.adjoint_directions;
             for (DevBuf* d : {&b->v, &b->gbx, &b->gby, &b->qbar, &b->u, &b->g, &b->q, &b->lam[0], &b->lam[1],
                               &b->ls[0], &b->ls[1]})
                 d->alloc(N * 32);

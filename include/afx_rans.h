@@ -93,9 +93,9 @@ int afx_config_from_ini_string(const char* text, afx_config* out);
  * loops, 0 = the same kernels driven from a host loop, for profilers) and
  * krylov_preconditioner (the flexible GMRES of afx_newton_solve and of the
  * implicit adjoint: 1 = a GMRES solve with the implicit matrix, 0 = one
- * ILU(0) sweep with it) and adjoint_directions (input directions per pass
- * of the vJP's face kernel, 1, 2 or 4: vector dual numbers that share the
- * value's work; every choice gives the same bits). */
+ * ILU(0) sweep with it) and adjoint_directions (1, 2 or 4, for callers
+ * that set it: the vJP's face kernel is one reverse sweep whatever the value,
+ * and every choice gives the same bits). */
 int afx_config_set_double(afx_config c, const char* key, double v);
 int afx_config_get_double(afx_config c, const char* key, double* v);
 /* String fields: solver ("explicit"/"implicit"), gradient ("green-gauss"/
