@@ -98,6 +98,13 @@ template <> struct Div<double> {
 };
 __device__ __forceinline__ double dabs(double x) { return fabs(x); }
 __device__ __forceinline__ float dabs(float x) { return fabsf(x); }
+// x or -x, without an FP64 instruction and without a branch around the sum it
+// goes into (a - b and a + (-b) are the same number; two branches of a sum are
+// formed one after the other in a warp whose lanes differ)
+__device__ __forceinline__ float flip(const float x, const bool neg) { return neg ? -x : x; }
+__device__ __forceinline__ double flip(const double x, const bool neg) {
+    return fp64::of_bits(fp64::bits_of(x) ^ (neg ? 0x8000000000000000ull : 0ull));
+}
 
 // std::min / std::max semantics: min(a,b) = (b < a) ? b : a; max(a,b) = (a < b) ? b : a
 template <class T> __device__ __forceinline__ T smin(T a, T b) { return (b < a) ? b : a; }
