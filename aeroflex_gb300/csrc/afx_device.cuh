@@ -38,6 +38,9 @@ template <> struct V4t<float> { using type = float4; };
 template <class T> using V2 = typename V2t<T>::type;
 template <class T> using V4 = typename V4t<T>::type;
 
+// cnbr of an empty slot (a triangle's fourth)
+constexpr int NO_NEIGHBOUR = (int)0x80000000;
+
 enum { BT_INTERNAL = 0, BT_FARFIELD = 1, BT_SLIP = 2, BT_WALL = 3, BT_INOUT = 4 };
 
 __device__ __forceinline__ void ld4(const d4* p, double* v) {
@@ -76,8 +79,22 @@ __device__ __forceinline__ void st4(d4* p, const double* v) {
     q[1] = make_double2(v[2], v[3]);
 }
 __device__ __forceinline__ void st4(float4* p, const float* v) { *p = make_float4(v[0], v[1], v[2], v[3]); }
+// conversions in integer arithmetic: the instructions hold the FP64 pipe
+__device__ __forceinline__ double to_f64(const float x) { return fp64::widen(__float_as_uint(x)); }
+__device__ __forceinline__ float to_f32(const double x) {
+    uint32_t r;
+    if (!fp64::narrow(x, r)) return (float)x;
+    return __uint_as_float(r);
+}
 __device__ __forceinline__ void st4(float4* p, const double* v) {
-    *p = make_float4((float)v[0], (float)v[1], (float)v[2], (float)v[3]);
+    *p = make_float4(to_f32(v[0]), to_f32(v[1]), to_f32(v[2]), to_f32(v[3]));
+}
+// (h, l) += (oh, ol), unevaluated pairs: Knuth's two-sum of the leading parts
+__device__ __forceinline__ void pair_add(float& h, float& l, const float oh, const float ol) {
+    const float s = __fadd_rn(h, oh), b = __fadd_rn(s, -h);
+    const float err = __fadd_rn(__fadd_rn(h, -__fadd_rn(s, -b)), __fadd_rn(oh, -b));
+    l = __fadd_rn(__fadd_rn(l, ol), err);
+    h = s;
 }
 
 __device__ __forceinline__ double dsqrt(double x) { return fp64::root(x); }
@@ -115,7 +132,8 @@ __device__ __forceinline__ double smax(double a, double b) { return fp64::less(a
 // Kernel view of the mesh and physics.
 template <class T>
 struct KM {
-    int n_cells;
+    int n_cells, n_faces;
+    int ahead;  // blocks ahead of the running one whose data is brought into L2 (0: none)
     const int4* __restrict__ cslot;  // +(face+1) if the cell is the face's cell 0, -(face+1) if cell 1, 0 empty
     const int4* __restrict__ cnbr;   // the face's other cell, or -(b+1) for boundary face b
     const T* __restrict__ area;
@@ -124,6 +142,7 @@ struct KM {
     const V2<T>* __restrict__ fLg;
     const V2<T>* __restrict__ fd0;
     const V2<T>* __restrict__ fd1;
+    const V2<T>* __restrict__ dsl;  // FP32: the cells' own offsets, slot s of cell i at s * n_cells + i
     const V4<T>* __restrict__ ft;
     const int* __restrict__ btype;
     const V4<T>* __restrict__ bq;

@@ -110,6 +110,26 @@ static double div_rare(const double x, const double y) { return x / y; }
 static double root_rare(const double x) { return __builtin_sqrt(x); }
 #endif
 
+// (double)x, FP32 subnormals as zero (as the FP32 kernels are compiled)
+AFX_HD double widen(const uint32_t u) {
+    const uint32_t e = (u >> 23) & 0xffu, mag = u & 0x7fffffffu;
+    const uint32_t hi = (mag >> 3) + (e == 0xffu ? 0x70000000u : 0x38000000u);
+    const uint64_t v = e == 0 ? 0ull : ((uint64_t)hi << 32) | (u << 29);
+    return of_bits(v | ((uint64_t)(u & 0x80000000u) << 32));
+}
+// bits of (float)x, round to nearest even; false outside FP32's normal range
+// (other than zero)
+AFX_HD bool narrow(const double x, uint32_t& r) {
+    const uint64_t u = bits_of(x);
+    const uint32_t hi = (uint32_t)(u >> 32), lo = (uint32_t)u, sgn = hi & 0x80000000u;
+    const uint32_t e = (hi >> 20) & 0x7ffu;
+    const uint32_t m = ((e - 896u) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29);
+    const uint32_t rem = lo & 0x1fffffffu;
+    r = (m + (rem + (m & 1u) > 0x10000000u ? 1u : 0u)) | sgn;
+    if ((hi << 1 | lo) == 0u) r = sgn;
+    return e - 897u < 254u || (hi << 1 | lo) == 0u;
+}
+
 // A denominator: its significand and a 32-bit reciprocal, shared by the
 // quotients that divide by it.
 struct Den {

@@ -120,7 +120,7 @@ struct DeviceLayout {
     std::vector<int32_t> cell_new;       // reference cell -> device cell
     std::vector<int32_t> face_edge;      // device face -> reference edge
     std::vector<int32_t> cslot;          // 4 per device cell: +-(device face + 1), 0 pad
-    std::vector<int32_t> cnbr;           // 4 per device cell: other cell or -(b+1)
+    std::vector<int32_t> cnbr;           // 4 per device cell: other cell or -(b+1); empty slot: INT32_MIN
     std::vector<int32_t> fcell;          // 2 per device face: c0, c1 (c1 < 0: boundary -(b+1))
     std::vector<double> area;            // per device cell
     std::vector<double> fn, fLg, fd0, fd1, ft;  // 2,2,2,2,4 per face
@@ -131,5 +131,8 @@ DeviceLayout build_layout(const HostMesh& m);
 // The geometric face and cell records of L (fn, fLg, fd0, fd1, ft, area) from
 // the metrics of m, keeping L's numbering.
 void fill_layout_geometry(const HostMesh& m, DeviceLayout& L);
+// Face centre minus centroid of each cell's slots, slot-major: (x, y) of slot s
+// of cell i at 2 (s N + i); zero in an empty slot.
+std::vector<float> slot_offsets(const DeviceLayout& L);
 
 }  // namespace afx

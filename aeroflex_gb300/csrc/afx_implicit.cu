@@ -739,12 +739,7 @@ template <> struct Part<float> {
         o.l = __shfl_xor_sync(0xffffffffu, l, m);
         return o;
     }
-    __device__ __forceinline__ void add(const Part& o) {  // Knuth's two-sum of the leading parts
-        const float s = __fadd_rn(h, o.h), b = __fadd_rn(s, -h);
-        const float err = __fadd_rn(__fadd_rn(h, -__fadd_rn(s, -b)), __fadd_rn(o.h, -b));
-        l = __fadd_rn(__fadd_rn(l, o.l), err);
-        h = s;
-    }
+    __device__ __forceinline__ void add(const Part& o) { pair_add(h, l, o.h, o.l); }
 };
 // Sums of acc[0..W-1] over the warp; lane j (mod W) gets output j
 template <int W, class T>

@@ -29,6 +29,15 @@ __device__ __forceinline__ void ld4p(const float4* p, float* v) {
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
 }
 
+// Elements [i, j) (clipped to n) of an array of `size`-byte elements into L2.
+__device__ __forceinline__ void l2_ahead(const void* base, const int size, const long long i, const long long j,
+                                         const long long n) {
+    const long long b = (i * size) & ~15ll, e = ((j < n ? j : n) * size) & ~15ll;
+    if (b < e)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;"
+                     :: "l"(reinterpret_cast<const char*>(base) + b), "r"((unsigned)(e - b)));
+}
+
 // The cell's limiter (solver.h:517-593): per variable the least limiter_value
 // over its faces, at most 1.  sl: the cell's slots (0: none); dx, dy: face
 // centre minus centroid per slot.
@@ -125,11 +134,23 @@ __device__ __forceinline__ void cell_limiter<double>(const KM<double>& m, const 
 // Green-Gauss gradient (solver.h:428-469) and, when second order, the first
 // stage's neighbour min/max and limiter (solver.h:517-593).
 template <class T, class S, bool GRAD, bool SECOND, bool DTP>
-__global__ void __launch_bounds__(256) k_prep(const KM<T> m, const V4<S>* __restrict__ q, V4<T>* __restrict__ gx,
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_prep(const KM<T> m, const V4<S>* __restrict__ q, V4<T>* __restrict__ gx,
                                               V4<T>* __restrict__ gy, V4<T>* __restrict__ phi,
                                               T* __restrict__ dt, const Ctrl* __restrict__ ctrl) {
     if (ctrl->done) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (sizeof(T) == 4 && m.ahead && threadIdx.x < 8) {
+        const long long b0 = (long long)(blockIdx.x + m.ahead) * blockDim.x, b1 = b0 + blockDim.x;
+        const long long f0 = b0 * m.n_faces / m.n_cells, f1 = b1 * m.n_faces / m.n_cells;
+        const int t = threadIdx.x;
+        if (t < 4) {
+            const void* a = t == 0 ? (const void*)m.cslot : t == 1 ? (const void*)m.cnbr : t == 2 ? (const void*)q : (const void*)m.area;
+            l2_ahead(a, t == 3 ? (int)sizeof(T) : 16, b0, b1, m.n_cells);
+        } else {
+            const void* a = t == 4 ? (const void*)m.fn : t == 5 ? (const void*)m.fLg : t == 6 ? (const void*)m.fd0 : (const void*)m.fd1;
+            l2_ahead(a, 2 * (int)sizeof(T), f0, f1, m.n_faces);
+        }
+    }
     if (i >= m.n_cells) return;
     const int4 sl = __ldg(&m.cslot[i]);
     const int4 nb = __ldg(&m.cnbr[i]);
@@ -330,6 +351,80 @@ __global__ void __launch_bounds__(256) k_limiter(const KM<T> m, const V4<S>* __r
     phi[i] = vp;
 }
 
+// The same in FP32: the offsets of a cell's face centres come from the cell's
+// own slots (m.dsl), side by side in a warp, in place of two gathers through the
+// face numbers; an empty slot is marked in cnbr.  Latency-bound (35% of DRAM
+// before): everything but the neighbours' states is a direct load, and the
+// streams of a block some way ahead are brought into L2.
+template <class S>
+__global__ void __launch_bounds__(256) k_limiter_f32(const KM<float> m, const V4<S>* __restrict__ qk,
+                                                     const float4* __restrict__ gx, const float4* __restrict__ gy,
+                                                     float4* __restrict__ phi, const Ctrl* __restrict__ ctrl) {
+    if (ctrl->done) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m.ahead && threadIdx.x < 8) {
+        const long long b0 = (long long)(blockIdx.x + m.ahead) * blockDim.x, b1 = b0 + blockDim.x, N = m.n_cells;
+        const int t = threadIdx.x;
+        if (t < 5) {
+            const void* a = t == 0 ? (const void*)m.cnbr
+                            : t == 1 ? (const void*)qk
+                            : t == 2 ? (const void*)gx
+                            : t == 3 ? (const void*)gy
+                                     : (const void*)m.area;
+            l2_ahead(a, t == 4 ? 4 : 16, b0, b1, N);
+        } else {
+            const long long o = (long long)(t - 5) * N;
+            l2_ahead(m.dsl, 8, o + b0, o + (b1 < N ? b1 : N), 4 * N);
+        }
+    }
+    if (i >= m.n_cells) return;
+    const int4 nb = __ldg(&m.cnbr[i]);
+    float qi[4], gxi[4], gyi[4];
+    ld4s(&qk[i], qi);
+    ld4c<float>(&gx[i], gxi);
+    ld4c<float>(&gy[i], gyi);
+    float dxs[4], dys[4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        float2 d = make_float2(0.f, 0.f);
+        if (s < 3 || nb.w != NO_NEIGHBOUR) d = __ldg(&m.dsl[(size_t)s * m.n_cells + i]);
+        dxs[s] = d.x;
+        dys[s] = d.y;
+    }
+    const float A = __ldg(&m.area[i]);
+    float qmn[4], qmx[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) qmn[k] = qmx[k] = qi[k];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        const int o = pick(nb, s);
+        if (o == NO_NEIGHBOUR) continue;
+        bool use = true;
+        float qo[4];
+        if (o >= 0) {
+            ld4s(&qk[o], qo);
+        } else {
+            const int bt = __ldg(&m.btype[-o - 1]);
+            use = bt != BT_SLIP && bt != BT_WALL;
+            ld4c<float>(&m.bq[-o - 1], qo);
+        }
+        if (use) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                qmn[k] = smin(qmn[k], qo[k]);
+                qmx[k] = smax(qmx[k], qo[k]);
+            }
+        }
+    }
+    const float sqrt_area = dsqrt(A);
+    const float Ka = m.limk * sqrt_area;
+    const float K3a = Ka * Ka * Ka;
+    float lim[4];
+    const int4 on = make_int4(nb.x != NO_NEIGHBOUR, nb.y != NO_NEIGHBOUR, nb.z != NO_NEIGHBOUR, nb.w != NO_NEIGHBOUR);
+    cell_limiter<float>(m, on, qi, qmn, qmx, gxi, gyi, dxs, dys, K3a, lim);
+    phi[i] = make_float4(lim[0], lim[1], lim[2], lim[3]);
+}
+
 // Second-order reconstruction of one side, solver.h:780-781:
 // q + (gx*dx + gy*dy) .* phi
 template <class T>
@@ -410,17 +505,38 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
     return t;
 }
 
+// The same over a block's FP32 values, as unevaluated pairs on the FP32 lanes
+// (the sum is good to 48 bits; shuffled doubles took five FP64 additions per
+// warp).  sh: 64 floats' worth.
+__device__ __forceinline__ double block_sum_f32(const float v, double* sh) {
+    float h = v, l = 0.f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        pair_add(h, l, __shfl_down_sync(0xffffffffu, h, o), __shfl_down_sync(0xffffffffu, l, o));
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    float2* s = reinterpret_cast<float2*>(sh);
+    if (lane == 0) s[w] = make_float2(h, l);
+    __syncthreads();
+    if (threadIdx.x != 0) return 0.0;
+    h = l = 0.f;
+    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) pair_add(h, l, s[k].x, s[k].y);
+    return (double)h + (double)l;
+}
+
 // FP32-mixed epilogue.  GB300's FP64 pipe issues at ~1/64 of the FP32 rate,
-// so FP64 is spent only where it accumulates: the RK increment
+// so FP64 is spent only where it accumulates, in the four additions to the state
+// (conversions are integer arithmetic, the norm's sum pairs of FP32: with both
+// on the FP64 pipe some 20 of its instructions per warp made the last stage
+// 220 us at 4.19M cells, 170 now): the RK increment
 // R*dt*alpha*relaxation is formed in FP32; the intermediate stage states
 // (which only feed FP32 fluxes) are q_shadow + increment in FP32; the new
 // state of the last stage is q (FP64) + increment in FP64, and its FP32
 // shadow is re-rounded from the FP64 result every iteration, so FP32
 // rounding never accumulates in the state.  The norm sums per-cell FP32
-// squares in FP64.
+// squares as unevaluated pairs in a block and in FP64 over the blocks.
 template <class S>
 __device__ __forceinline__ void stage_epilogue_mixed(const StageOut<float, S>& o, const int i, const float* R0,
-                                                     const float dti, double& sq) {
+                                                     const float dti, float& sq) {
     // defect correction: R = R32(q) + (R64 - R32)(q_ref), see k_correction
     float R[4] = {R0[0], R0[1], R0[2], R0[3]};
     if (o.corr) {
@@ -445,24 +561,25 @@ __device__ __forceinline__ void stage_epilogue_mixed(const StageOut<float, S>& o
         ld4(&o.q0[i], q0);
         double qn[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) qn[k] = q0[k] + (double)inc[k];
+        for (int k = 0; k < 4; ++k) qn[k] = q0[k] + to_f64(inc[k]);
         st4(&o.qm_next[i], qn);
         if (o.qsh_next) {
             V4<S> v;
             st4(&v, qn);
             o.qsh_next[i] = v;
         }
-        sq += (double)(R[0] * R[0] + R[1] * R[1] + R[2] * R[2] + R[3] * R[3]);
+        sq = R[0] * R[0] + R[1] * R[1] + R[2] * R[2] + R[3] * R[3];
     }
 }
 template <class S>
 __device__ __forceinline__ void stage_epilogue_mixed(const StageOut<double, S>&, const int, const double*,
-                                                     const double, double&) {}
+                                                     const double, float&) {}
 
 template <class T, class S>
 __device__ __forceinline__ void stage_epilogue(const StageOut<T, S>& o, const int i, const bool active, const T* Rsum,
                                                const T A, const T dti, const double extra_sq, double* sh) {
     double sq = extra_sq;
+    float sqf = 0.f;  // FP32: the cell's square
     if (active) {
         T R[4];
         const Div<T> iA(A);
@@ -509,7 +626,7 @@ __device__ __forceinline__ void stage_epilogue(const StageOut<T, S>& o, const in
             for (int k = 0; k < 4; ++k) sq += Rd[k] * Rd[k];
             if (o.cell_sq) o.cell_sq[i] = sq;
         } else if (sizeof(T) == 4) {
-            stage_epilogue_mixed<S>(o, i, R, dti, sq);
+            stage_epilogue_mixed<S>(o, i, R, dti, sqf);
         } else {
             double q0[4];
             ld4(&o.q0[i], q0);
@@ -536,12 +653,22 @@ __device__ __forceinline__ void stage_epilogue(const StageOut<T, S>& o, const in
         if (o.cell_sq && o.mode == 1 && !(o.case_done && __ldg(&o.case_done[__ldg(&o.case_of[i])]))) {
             // batch: the last stage's qW stays in Rq for a later
             // get_uniform_residual (each case stops at its own iteration)
-            o.cell_sq[i] = sq;
-            double Rd[4] = {(double)R[0], (double)R[1], (double)R[2], (double)R[3]};
-            st4(&o.Rq[i], Rd);
+            if constexpr (sizeof(T) == 4) {
+                o.cell_sq[i] = fp64::bits_of(sq) ? sq + (double)sqf : to_f64(sqf);
+                double Rd[4] = {to_f64(R[0]), to_f64(R[1]), to_f64(R[2]), to_f64(R[3])};
+                st4(&o.Rq[i], Rd);
+            } else {
+                o.cell_sq[i] = sq;
+                double Rd[4] = {R[0], R[1], R[2], R[3]};
+                st4(&o.Rq[i], Rd);
+            }
         }
     }
-    if (o.mode == 1 || o.mode == 3) {
+    if (sizeof(T) == 4 && o.mode == 1 && !__syncthreads_or(fp64::bits_of(sq) != 0)) {
+        const double t = block_sum_f32(sqf, sh);
+        if (threadIdx.x == 0) o.partials[blockIdx.x] = t;
+    } else if (o.mode == 1 || o.mode == 3) {
+        if (sizeof(T) == 4) sq += (double)sqf;  // with the squares of frozen ghosts
         const double t = block_sum(sq, sh);
         if (threadIdx.x == 0) o.partials[blockIdx.x] = t;
     }
@@ -788,8 +915,14 @@ struct TileView {
     const short4* __restrict__ ctile;  // per cell: +-(tile-local face + 1) per slot, edge order
 };
 
+//
+// Registers (FP32): 32 without a viscous term, so eight blocks are resident; the
+// kernel is bound by latency and more warps hide it better than more loads per
+// warp (4.19M cells: 167 us a stage, with 40 registers 187).  The viscous terms
+// need more than twice as many and spilled 250 bytes per thread at 32 (17k
+// cells: 8.9 -> 6.8 us at 80).
 template <class T, class S, int VISC, bool SECOND, bool EIG>
-__global__ void __launch_bounds__(256, 8) k_resid_tile(const KM<T> m, const TileView tv, const V4<S>* __restrict__ qk,
+__global__ void __launch_bounds__(256, VISC == 0 ? 8 : 3) k_resid_tile(const KM<T> m, const TileView tv, const V4<S>* __restrict__ qk,
                                                     const V4<S>* __restrict__ qmem, const V4<T>* __restrict__ gx,
                                                     const V4<T>* __restrict__ gy, const V4<T>* __restrict__ phi,
                                                     const StageOut<T, S> o, const Ctrl* __restrict__ ctrl) {

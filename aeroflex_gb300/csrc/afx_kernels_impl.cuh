@@ -12,6 +12,13 @@ template <class T>
 KM<T> make_km(const StepArgs& a) {
     KM<T> m;
     m.n_cells = a.n_cells;
+    m.n_faces = a.n_faces;
+    // the streams of a block two blocks per SM on are brought into L2 (k_prep
+    // 173 -> 154 us, k_limiter_f32 85 -> 79 us at 4.19M cells; four per SM no
+    // better, eight worse); below about a million cells the arrays stay in L2 by
+    // themselves and the requests only cost time (k_limiter, 590k cells: 15.9 ->
+    // 16.8 us)
+    m.ahead = a.n_cells >= 1000000 ? 304 : 0;
     m.cslot = (const int4*)a.cslot;
     m.cnbr = (const int4*)a.cnbr;
     m.area = (const T*)a.area;
@@ -20,6 +27,7 @@ KM<T> make_km(const StepArgs& a) {
     m.fLg = (const V2<T>*)a.fLg;
     m.fd0 = (const V2<T>*)a.fd0;
     m.fd1 = (const V2<T>*)a.fd1;
+    m.dsl = (const V2<T>*)a.dsl;
     m.ft = (const V4<T>*)a.ft;
     m.btype = (const int*)a.btype;
     m.bq = (const V4<T>*)a.bq;
@@ -203,8 +211,13 @@ void iteration(const StepArgs& a, int p, cudaStream_t s) {
     for (int st = 0; st < 3; ++st) {
         const V4<S>* qk = st == 0 ? q : (const V4<S>*)a.qs[st - 1];
         if (st > 0 && a.second) {
-            k_limiter<T, S><<<nblocks(a.n_cells, a.block), a.block, 0, s>>>(
-                m, qk, (const V4<T>*)a.gx, (const V4<T>*)a.gy, (V4<T>*)a.phi, a.ctrl);
+            const int nl = nblocks(a.n_cells, a.block);
+            if constexpr (sizeof(T) == 4)
+                k_limiter_f32<S><<<nl, a.block, 0, s>>>(m, qk, (const V4<T>*)a.gx, (const V4<T>*)a.gy, (V4<T>*)a.phi,
+                                                        a.ctrl);
+            else
+                k_limiter<T, S><<<nl, a.block, 0, s>>>(m, qk, (const V4<T>*)a.gx, (const V4<T>*)a.gy, (V4<T>*)a.phi,
+                                                       a.ctrl);
             mark(a, K_LIMITER, s);
         }
         // Spalart-Allmaras: eddy viscosity of the stage state first

@@ -68,6 +68,7 @@ struct StepArgs {
     const void* fd0 = nullptr;    // T2 [F]
     const void* fd1 = nullptr;    // T2 [F]
     const void* ft = nullptr;     // T4 [F]
+    const void* dsl = nullptr;    // T2 [4N] (FP32): face centre - centroid per cell slot, slot-major
     const void* btype = nullptr;  // int [B]
     const void* bq = nullptr;     // T4 [B] ghost (boundary) states
     // physics / scheme

@@ -501,7 +501,7 @@ DeviceLayout build_layout(const HostMesh& m) {
     // cell is the face's cell 0, -(face+1) when it is cell 1; the other cell
     // (device id, or -(b+1) for boundary b) beside it
     L.cslot.assign(4 * (size_t)N, 0);
-    L.cnbr.assign(4 * (size_t)N, 0);
+    L.cnbr.assign(4 * (size_t)N, INT32_MIN);
     std::vector<uint8_t> cnt(N, 0);
     for (int e = 0; e < E; ++e) {
         const uint32_t c0 = m.edgesCells[e][0], c1 = m.edgesCells[e][1];
@@ -572,6 +572,22 @@ void fill_layout_geometry(const HostMesh& m, DeviceLayout& L) {
     }
     L.area.assign(N, 0.);
     for (int i = 0; i < N; ++i) L.area[i] = m.cellsAreas[L.cell_old[i]];
+}
+
+std::vector<float> slot_offsets(const DeviceLayout& L) {
+    const size_t N = L.n_cells;
+    std::vector<float> d(8 * N, 0.f);
+#pragma omp parallel for
+    for (long i = 0; i < (long)N; ++i)
+        for (int s = 0; s < 4; ++s) {
+            const int v = L.cslot[4 * i + s];
+            if (v == 0) continue;
+            const size_t f = (v > 0 ? v : -v) - 1;
+            const std::vector<double>& fd = v > 0 ? L.fd0 : L.fd1;
+            d[2 * (s * N + i)] = (float)fd[2 * f];
+            d[2 * (s * N + i) + 1] = (float)fd[2 * f + 1];
+        }
+    return d;
 }
 
 }  // namespace afx
