@@ -2208,13 +2208,13 @@ int afx_batch_set_state(afx_batch b, int c, const double* q, long long n) {
         if (!b || !q) throw Error(AFX_ERR_ARG, "null argument");
         b->check_case(c);
         afx_solver_s& s = *b->s;
-        const size_t N = s.a.n_cells, c0 = b->cell_off[c], nc = b->cell_off[c + 1] - c0;
+        const size_t c0 = b->cell_off[c], nc = b->cell_off[c + 1] - c0;
         if (n != (long long)(4 * nc)) throw Error(AFX_ERR_ARG, "state size must be 4*n_real_cells of the case");
-        // whole state out in reference order, the case's slice replaced, back in
-        enqueue_permute_out((int)N, (const int*)s.d_cell_old.p, s.a.qm[s.parity], s.d_stage.p, s.stream);
+        // a case's cells are one range in both orders: only that range moves
         AFX_CUDA(cudaMemcpyAsync((double*)s.d_stage.p + 4 * c0, q, nc * 32, cudaMemcpyDefault, s.stream));
-        enqueue_permute_in((int)N, (const int*)s.d_cell_old.p, s.d_stage.p, s.a.qm[s.parity], s.stream);
-        s.sync_shadow(s.parity);
+        double* qm = (double*)s.a.qm[s.parity] + 4 * c0;
+        enqueue_permute_in((int)nc, (const int*)s.d_cell_old.p + c0, s.d_stage.p, qm, s.stream);
+        if (!s.fp64) enqueue_to_f32((int)nc, qm, (float*)s.a.qsh[s.parity] + 4 * c0, s.stream);
         AFX_CUDA(cudaStreamSynchronize(s.stream));
     });
 }
@@ -2224,9 +2224,10 @@ int afx_batch_get_state(afx_batch b, int c, double* q, long long n) {
         if (!b || !q) throw Error(AFX_ERR_ARG, "null argument");
         b->check_case(c);
         afx_solver_s& s = *b->s;
-        const size_t N = s.a.n_cells, c0 = b->cell_off[c], nc = b->cell_off[c + 1] - c0;
+        const size_t c0 = b->cell_off[c], nc = b->cell_off[c + 1] - c0;
         if (n != (long long)(4 * nc)) throw Error(AFX_ERR_ARG, "state size must be 4*n_real_cells of the case");
-        enqueue_permute_out((int)N, (const int*)s.d_cell_old.p, s.a.qm[s.parity], s.d_stage.p, s.stream);
+        enqueue_permute_out((int)nc, (const int*)s.d_cell_old.p + c0, (const double*)s.a.qm[s.parity] + 4 * c0,
+                            s.d_stage.p, s.stream);
         AFX_CUDA(cudaMemcpyAsync(q, (const double*)s.d_stage.p + 4 * c0, nc * 32, cudaMemcpyDefault, s.stream));
         AFX_CUDA(cudaStreamSynchronize(s.stream));
     });

@@ -9,7 +9,10 @@
 // loads of all faces of a cell are in flight together.
 #pragma once
 
+#include <cooperative_groups.h>
+
 #include "afx_device.cuh"
+#include "afx_pdl.cuh"
 
 namespace afx {
 namespace dev {
@@ -26,6 +29,17 @@ __device__ __forceinline__ void ld4p(const d4* p, double* v) {
 }
 __device__ __forceinline__ void ld4p(const float4* p, float* v) {
     const float4 a = *p;
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+}
+
+// Loads of what the kernel launched just before may have written (afx_pdl.cuh)
+__device__ __forceinline__ void ldw4(const d4* p, double* v) {
+    const double2* q = reinterpret_cast<const double2*>(p);
+    const double2 a = ldw(q), b = ldw(q + 1);
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+__device__ __forceinline__ void ldw4(const float4* p, float* v) {
+    const float4 a = ldw(p);
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
 }
 
@@ -134,10 +148,9 @@ __device__ __forceinline__ void cell_limiter<double>(const KM<double>& m, const 
 // Green-Gauss gradient (solver.h:428-469) and, when second order, the first
 // stage's neighbour min/max and limiter (solver.h:517-593).
 template <class T, class S, bool GRAD, bool SECOND, bool DTP>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_prep(const KM<T> m, const V4<S>* __restrict__ q, V4<T>* __restrict__ gx,
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_prep(const KM<T> m, const V4<S>* __restrict__ q, V4<T>* __restrict__ gx,
                                               V4<T>* __restrict__ gy, V4<T>* __restrict__ phi,
                                               T* __restrict__ dt, const Ctrl* __restrict__ ctrl) {
-    if (ctrl->done) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (sizeof(T) == 4 && m.ahead && threadIdx.x < 8) {
         const long long b0 = (long long)(blockIdx.x + m.ahead) * blockDim.x, b1 = b0 + blockDim.x;
@@ -151,11 +164,17 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_prep(const KM<T
             l2_ahead(a, 2 * (int)sizeof(T), f0, f1, m.n_faces);
         }
     }
-    if (i >= m.n_cells) return;
-    const int4 sl = __ldg(&m.cslot[i]);
-    const int4 nb = __ldg(&m.cnbr[i]);
+    int4 sl = make_int4(0, 0, 0, 0), nb = sl;
+    T A = T(1);
+    if (i < m.n_cells) {
+        sl = __ldg(&m.cslot[i]);
+        nb = __ldg(&m.cnbr[i]);
+        A = __ldg(&m.area[i]);
+    }
+    pdl_wait();
+    if (i >= m.n_cells || ldw(&ctrl->done)) return;
     T qi[4];
-    ld4s(&q[i], qi);
+    ldw4(&q[i], qi);
     T sgx[4] = {T(0), T(0), T(0), T(0)}, sgy[4] = {T(0), T(0), T(0), T(0)};
     T qmn[4], qmx[4];
 #pragma unroll
@@ -176,7 +195,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_prep(const KM<T
             T qo[4];
             int bt = BT_INTERNAL;
             if (o >= 0) {
-                ld4s(&q[o], qo);
+                ldw4(&q[o], qo);
             } else {
                 bt = __ldg(&m.btype[-o - 1]);
                 ld4c<T>(&m.bq[-o - 1], qo);
@@ -232,7 +251,6 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_prep(const KM<T
             }
         }
     }
-    const T A = __ldg(&m.area[i]);
     if (DTP) dt[i] = fdiv(m.cfl * A, eigsum);
     if (!GRAD) return;
     T gxi[4], gyi[4];
@@ -253,7 +271,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_prep(const KM<T
             T qo[4], qR[4];
             int bt = BT_INTERNAL;
             if (o >= 0) {
-                ld4s(&q[o], qo);
+                ldw4(&q[o], qo);
             } else {
                 bt = __ldg(&m.btype[-o - 1]);
                 ld4c<T>(&m.bq[-o - 1], qo);
@@ -297,15 +315,21 @@ template <class T, class S>
 __global__ void __launch_bounds__(256) k_limiter(const KM<T> m, const V4<S>* __restrict__ qk,
                                                  const V4<T>* __restrict__ gx, const V4<T>* __restrict__ gy,
                                                  V4<T>* __restrict__ phi, const Ctrl* __restrict__ ctrl) {
-    if (ctrl->done) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m.n_cells) return;
-    const int4 sl = __ldg(&m.cslot[i]);
-    const int4 nb = __ldg(&m.cnbr[i]);
-    T qi[4], gxi[4], gyi[4];
-    ld4s(&qk[i], qi);
-    ld4c<T>(&gx[i], gxi);
-    ld4c<T>(&gy[i], gyi);
+    // the gradients are the iteration's, complete before the stage kernel that
+    // this one follows
+    int4 sl = make_int4(0, 0, 0, 0), nb = sl;
+    T A = T(1), qi[4], gxi[4], gyi[4];
+    if (i < m.n_cells) {
+        sl = __ldg(&m.cslot[i]);
+        nb = __ldg(&m.cnbr[i]);
+        A = __ldg(&m.area[i]);
+        ld4c<T>(&gx[i], gxi);
+        ld4c<T>(&gy[i], gyi);
+    }
+    pdl_wait();
+    if (i >= m.n_cells || ldw(&ctrl->done)) return;
+    ldw4(&qk[i], qi);
     T qmn[4], qmx[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) { qmn[k] = qi[k]; qmx[k] = qi[k]; }
@@ -325,7 +349,7 @@ __global__ void __launch_bounds__(256) k_limiter(const KM<T> m, const V4<S>* __r
             bool use = true;
             T qo[4];
             if (o >= 0) {
-                ld4s(&qk[o], qo);
+                ldw4(&qk[o], qo);
             } else {
                 const int bt = __ldg(&m.btype[-o - 1]);
                 use = bt != BT_SLIP && bt != BT_WALL;
@@ -340,7 +364,6 @@ __global__ void __launch_bounds__(256) k_limiter(const KM<T> m, const V4<S>* __r
             }
         }
     }
-    const T A = __ldg(&m.area[i]);
     const T sqrt_area = dsqrt(A);
     const T Ka = m.limk * sqrt_area;
     const T K3a = Ka * Ka * Ka;
@@ -360,7 +383,6 @@ template <class S>
 __global__ void __launch_bounds__(256) k_limiter_f32(const KM<float> m, const V4<S>* __restrict__ qk,
                                                      const float4* __restrict__ gx, const float4* __restrict__ gy,
                                                      float4* __restrict__ phi, const Ctrl* __restrict__ ctrl) {
-    if (ctrl->done) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (m.ahead && threadIdx.x < 8) {
         const long long b0 = (long long)(blockIdx.x + m.ahead) * blockDim.x, b1 = b0 + blockDim.x, N = m.n_cells;
@@ -377,21 +399,25 @@ __global__ void __launch_bounds__(256) k_limiter_f32(const KM<float> m, const V4
             l2_ahead(m.dsl, 8, o + b0, o + (b1 < N ? b1 : N), 4 * N);
         }
     }
-    if (i >= m.n_cells) return;
-    const int4 nb = __ldg(&m.cnbr[i]);
-    float qi[4], gxi[4], gyi[4];
-    ld4s(&qk[i], qi);
-    ld4c<float>(&gx[i], gxi);
-    ld4c<float>(&gy[i], gyi);
-    float dxs[4], dys[4];
+    // all but the states is complete before the stage kernel that this one follows
+    int4 nb = make_int4(0, 0, 0, 0);
+    float qi[4], gxi[4], gyi[4], dxs[4], dys[4], A = 1.f;
+    if (i < m.n_cells) {
+        nb = __ldg(&m.cnbr[i]);
+        ld4c<float>(&gx[i], gxi);
+        ld4c<float>(&gy[i], gyi);
 #pragma unroll
-    for (int s = 0; s < 4; ++s) {
-        float2 d = make_float2(0.f, 0.f);
-        if (s < 3 || nb.w != NO_NEIGHBOUR) d = __ldg(&m.dsl[(size_t)s * m.n_cells + i]);
-        dxs[s] = d.x;
-        dys[s] = d.y;
+        for (int s = 0; s < 4; ++s) {
+            float2 d = make_float2(0.f, 0.f);
+            if (s < 3 || nb.w != NO_NEIGHBOUR) d = __ldg(&m.dsl[(size_t)s * m.n_cells + i]);
+            dxs[s] = d.x;
+            dys[s] = d.y;
+        }
+        A = __ldg(&m.area[i]);
     }
-    const float A = __ldg(&m.area[i]);
+    pdl_wait();
+    if (i >= m.n_cells || ldw(&ctrl->done)) return;
+    ldw4(&qk[i], qi);
     float qmn[4], qmx[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) qmn[k] = qmx[k] = qi[k];
@@ -402,7 +428,7 @@ __global__ void __launch_bounds__(256) k_limiter_f32(const KM<float> m, const V4
         bool use = true;
         float qo[4];
         if (o >= 0) {
-            ld4s(&qk[o], qo);
+            ldw4(&qk[o], qo);
         } else {
             const int bt = __ldg(&m.btype[-o - 1]);
             use = bt != BT_SLIP && bt != BT_WALL;
@@ -797,43 +823,56 @@ __global__ void __launch_bounds__(256) k_resid_gather(const KM<T> m, const V4<S>
 // face's spectral radius times length for the time step (solver.h:313-350).
 // The ghost side of a boundary face is its stored boundary state (ghost
 // gradients are zero).  Returns the face's boundary type in *btp.
+// g: the face's mesh records, which can be read before pdl_wait().
+template <class T, bool SECOND>
+struct FaceGeo {
+    int2 cc;
+    V2<T> n, d0, d1;
+    T L;
+    __device__ __forceinline__ void load(const KM<T>& m, const int f) {
+        cc = __ldg(&m.fcell[f]);
+        n = __ldg(&m.fn[f]);
+        L = __ldg(&m.fLg[f]).x;
+        if (SECOND) {
+            d0 = __ldg(&m.fd0[f]);
+            d1 = __ldg(&m.fd1[f]);
+        }
+    }
+};
 template <class T, class S, int VISC, bool SECOND, bool EIG>
-__device__ __forceinline__ void face_flux_at(const KM<T>& m, const int f, const V4<S>* __restrict__ qk,
-                                             const V4<S>* __restrict__ qmem, const V4<T>* __restrict__ gx,
-                                             const V4<T>* __restrict__ gy, const V4<T>* __restrict__ phi, T* fl,
-                                             T* eLp, int* btp) {
-    const int2 cc = __ldg(&m.fcell[f]);
-    const V2<T> n = __ldg(&m.fn[f]);
-    const T L = __ldg(&m.fLg[f]).x;
+__device__ __forceinline__ void face_flux_at(const KM<T>& m, const int f, const FaceGeo<T, SECOND>& g,
+                                             const V4<S>* qk, const V4<S>* qmem, const V4<T>* gx, const V4<T>* gy,
+                                             const V4<T>* phi, T* fl, T* eLp, int* btp) {
+    const int2 cc = g.cc;
+    const V2<T> n = g.n;
+    const T L = g.L;
     T q0[4], q1[4], qL[4], qR[4];
     T gx0[4] = {T(0), T(0), T(0), T(0)}, gy0[4] = {T(0), T(0), T(0), T(0)};
     T gx1[4] = {T(0), T(0), T(0), T(0)}, gy1[4] = {T(0), T(0), T(0), T(0)};
-    ld4s(&qk[cc.x], q0);
+    ldw4(&qk[cc.x], q0);
     if (SECOND || VISC >= 1) {
-        ld4c<T>(&gx[cc.x], gx0);
-        ld4c<T>(&gy[cc.x], gy0);
+        ldw4(&gx[cc.x], gx0);
+        ldw4(&gy[cc.x], gy0);
     }
     int bt = BT_INTERNAL;
     if (SECOND) {
         T p0[4];
-        ld4c<T>(&phi[cc.x], p0);
-        const V2<T> d0 = __ldg(&m.fd0[f]);
-        reconstruct(q0, gx0, gy0, p0, d0.x, d0.y, qL);
+        ldw4(&phi[cc.x], p0);
+        reconstruct(q0, gx0, gy0, p0, g.d0.x, g.d0.y, qL);
     } else {
 #pragma unroll
         for (int k = 0; k < 4; ++k) qL[k] = q0[k];
     }
     if (cc.y >= 0) {
-        ld4s(&qk[cc.y], q1);
+        ldw4(&qk[cc.y], q1);
         if (SECOND || VISC >= 1) {
-            ld4c<T>(&gx[cc.y], gx1);
-            ld4c<T>(&gy[cc.y], gy1);
+            ldw4(&gx[cc.y], gx1);
+            ldw4(&gy[cc.y], gy1);
         }
         if (SECOND) {
             T p1[4];
-            ld4c<T>(&phi[cc.y], p1);
-            const V2<T> d1 = __ldg(&m.fd1[f]);
-            reconstruct(q1, gx1, gy1, p1, d1.x, d1.y, qR);
+            ldw4(&phi[cc.y], p1);
+            reconstruct(q1, gx1, gy1, p1, g.d1.x, g.d1.y, qR);
         } else {
 #pragma unroll
             for (int k = 0; k < 4; ++k) qR[k] = q1[k];
@@ -858,8 +897,8 @@ __device__ __forceinline__ void face_flux_at(const KM<T>& m, const int f, const 
     T fgx[4] = {T(0), T(0), T(0), T(0)}, fgy[4] = {T(0), T(0), T(0), T(0)};
     if (VISC >= 1 && two_sided(bt)) {
         T qa[4], qb[4];
-        ld4s(&qmem[cc.x], qa);
-        if (cc.y >= 0) ld4s(&qmem[cc.y], qb);
+        ldw4(&qmem[cc.x], qa);
+        if (cc.y >= 0) ldw4(&qmem[cc.y], qb);
         else ld4c<T>(&m.bq[-cc.y - 1], qb);
         face_gradient(qa, qb, gx0, gy0, gx1, gy1, ldv4<T>(&m.ft[f]), fgx, fgy);
     }
@@ -884,17 +923,18 @@ __device__ __forceinline__ void face_flux_at(const KM<T>& m, const int f, const 
 // per face instead of once per cell side).  With EIG (first stage) it also
 // stores eig*L per face for the time step.
 template <class T, class S, int VISC, bool SECOND, bool EIG>
-__global__ void __launch_bounds__(256) k_face_flux(const KM<T> m, const int n_faces, const V4<S>* __restrict__ qk,
-                                                   const V4<S>* __restrict__ qmem, const V4<T>* __restrict__ gx,
-                                                   const V4<T>* __restrict__ gy, const V4<T>* __restrict__ phi,
-                                                   V4<T>* __restrict__ fflux, T* __restrict__ feL,
+__global__ void __launch_bounds__(256) k_face_flux(const KM<T> m, const int n_faces, const V4<S>* qk,
+                                                   const V4<S>* qmem, const V4<T>* gx, const V4<T>* gy,
+                                                   const V4<T>* phi, V4<T>* __restrict__ fflux, T* __restrict__ feL,
                                                    const Ctrl* __restrict__ ctrl) {
-    if (ctrl->done) return;
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= n_faces) return;
+    FaceGeo<T, SECOND> g;
+    if (f < n_faces) g.load(m, f);
+    pdl_wait();
+    if (f >= n_faces || ldw(&ctrl->done)) return;
     T fl[4], eL = T(0);
     int bt;
-    face_flux_at<T, S, VISC, SECOND, EIG>(m, f, qk, qmem, gx, gy, phi, fl, &eL, &bt);
+    face_flux_at<T, S, VISC, SECOND, EIG>(m, f, g, qk, qmem, gx, gy, phi, fl, &eL, &bt);
     V4<T> v;
     st4(&v, fl);
     fflux[f] = v;
@@ -922,24 +962,34 @@ struct TileView {
 // need more than twice as many and spilled 250 bytes per thread at 32 (17k
 // cells: 8.9 -> 6.8 us at 80).
 template <class T, class S, int VISC, bool SECOND, bool EIG>
-__global__ void __launch_bounds__(256, VISC == 0 ? 8 : 3) k_resid_tile(const KM<T> m, const TileView tv, const V4<S>* __restrict__ qk,
-                                                    const V4<S>* __restrict__ qmem, const V4<T>* __restrict__ gx,
-                                                    const V4<T>* __restrict__ gy, const V4<T>* __restrict__ phi,
+__global__ void __launch_bounds__(256, sizeof(T) == 8 ? 2 : (VISC == 0 ? 8 : 3)) k_resid_tile(const KM<T> m, const TileView tv, const V4<S>* qk,
+                                                    const V4<S>* qmem, const V4<T>* gx, const V4<T>* gy, const V4<T>* phi,
                                                     const StageOut<T, S> o, const Ctrl* __restrict__ ctrl) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ double sh[32];
-    if (ctrl->done) return;
     const int tile = blockIdx.x;
     const int h0 = __ldg(&tv.hstart[tile]), nh = __ldg(&tv.hstart[tile + 1]) - h0;
     const int x0 = __ldg(&tv.xptr[tile]), nf = nh + __ldg(&tv.xptr[tile + 1]) - x0;
     V4<T>* sF = reinterpret_cast<V4<T>*>(smem_raw);  // nf face fluxes F*L
     T* sE = reinterpret_cast<T*>(sF + nf);            // nf eig*L (EIG)
     double extra = 0;
+    FaceGeo<T, SECOND> g;
+    int f = 0;
+    constexpr bool FIRST = sizeof(T) == 8 || VISC > 0;  // the first face ahead of the wait (not at 32 registers)
+    if (FIRST && (int)threadIdx.x < nf) {
+        f = (int)threadIdx.x < nh ? h0 + threadIdx.x : __ldg(&tv.xlist[x0 + threadIdx.x - nh]);
+        g.load(m, f);
+    }
+    pdl_wait();
+    if (ldw(&ctrl->done)) return;
     for (int j = threadIdx.x; j < nf; j += blockDim.x) {
-        const int f = j < nh ? h0 + j : __ldg(&tv.xlist[x0 + j - nh]);
+        if (!FIRST || j != (int)threadIdx.x) {
+            f = j < nh ? h0 + j : __ldg(&tv.xlist[x0 + j - nh]);
+            g.load(m, f);
+        }
         T fl[4], eL = T(0);
         int bt;
-        face_flux_at<T, S, VISC, SECOND, EIG>(m, f, qk, qmem, gx, gy, phi, fl, &eL, &bt);
+        face_flux_at<T, S, VISC, SECOND, EIG>(m, f, g, qk, qmem, gx, gy, phi, fl, &eL, &bt);
         st4(&sF[j], fl);
         if (EIG) sE[j] = eL;
         if (o.mode == 1 && bt >= 0 && two_sided(bt))  // qW of a frozen ghost (solver.h:789-790)
@@ -981,19 +1031,22 @@ __global__ void __launch_bounds__(256, VISC == 0 ? 8 : 3) k_resid_tile(const KM<
 // With DT (first stage) the local time step dt = cfl*A/sum(eig*L) is formed
 // here from the face kernel's eig*L, in edge order, and stored.
 template <class T, class S, bool DT>
-__global__ void __launch_bounds__(256) k_cell_sum(const KM<T> m, const V4<T>* __restrict__ fflux,
-                                                  const T* __restrict__ feL, const StageOut<T, S> o,
+__global__ void __launch_bounds__(256) k_cell_sum(const KM<T> m, const V4<T>* fflux, const T* feL, const StageOut<T, S> o,
                                                   const Ctrl* __restrict__ ctrl) {
     __shared__ double sh[32];
-    if (ctrl->done) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool active = i < m.n_cells;
+    int4 sl = make_int4(0, 0, 0, 0), nb = sl;
+    if (active) {
+        sl = __ldg(&m.cslot[i]);
+        nb = __ldg(&m.cnbr[i]);
+    }
+    pdl_wait();
+    if (ldw(&ctrl->done)) return;
     T Rs[4] = {T(0), T(0), T(0), T(0)};
     double extra = 0;
     T A = T(1), dti = T(0);
     if (active) {
-        const int4 sl = __ldg(&m.cslot[i]);
-        const int4 nb = __ldg(&m.cnbr[i]);
         T eigsum = T(0);
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
@@ -1002,8 +1055,8 @@ __global__ void __launch_bounds__(256) k_cell_sum(const KM<T> m, const V4<T>* __
                 const bool own0 = fs > 0;
                 const int f = (own0 ? fs : -fs) - 1;
                 T fl[4];
-                ld4c<T>(&fflux[f], fl);
-                if (DT) eigsum += __ldg(&feL[f]);
+                ldw4(&fflux[f], fl);
+                if (DT) eigsum += ldw(&feL[f]);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) Rs[k] += flip(fl[k], own0);
                 const int oc = pick(nb, s);
@@ -1114,39 +1167,53 @@ __global__ void __launch_bounds__(256) k_uniform(const KM<T> m, const V4<S>* __r
     if (threadIdx.x == 0) partials[blockIdx.x] = t;
 }
 
-// Per-case norm and run_solver control of a batch (multigrid.h:195-234 for
-// every case): one block per case sums the per-cell squares of its cells in
-// a fixed order.  A case that stops is marked in case_done (its cells then
-// hold their state); the whole run stops when every case has.
-// Sum of cell_sq over [b0, b1) by one block: four accumulators per thread
-// (several loads in flight), then the fixed-order block sum.
-__device__ __forceinline__ double case_sum(const double* __restrict__ cell_sq, const int b0, const int b1,
-                                           double* sh) {
-    const int st = blockDim.x;
+// Sum of cell_sq over the cells [b0, b1) of a case by one cluster of CASE_CTAS
+// blocks (an FP64 sum of 60,000 cells holds the two FP64 lanes of a single SM
+// for 18 us; one block per case took 22): every block its share, four
+// accumulators per thread (several loads in flight), a fixed-order block sum,
+// then the blocks' sums in order.  Thread 0 of every block gets the total.
+constexpr int CASE_CTAS = 8, CASE_THREADS = 256;
+__device__ __forceinline__ double case_sum(const double* cell_sq, const int b0, const int b1, double* sh,
+                                           double* parts) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = (int)cl.block_rank(), share = (b1 - b0 + CASE_CTAS - 1) / CASE_CTAS;
+    const int e = min(b1, b0 + (rank + 1) * share), st = blockDim.x;
     double v0 = 0, v1 = 0, v2 = 0, v3 = 0;
-    int k = b0 + threadIdx.x;
-    for (; k + 3 * st < b1; k += 4 * st) {
-        v0 += cell_sq[k];
-        v1 += cell_sq[k + st];
-        v2 += cell_sq[k + 2 * st];
-        v3 += cell_sq[k + 3 * st];
+    int k = b0 + rank * share + threadIdx.x;
+    for (; k + 3 * st < e; k += 4 * st) {
+        v0 += ldw(&cell_sq[k]);
+        v1 += ldw(&cell_sq[k + st]);
+        v2 += ldw(&cell_sq[k + 2 * st]);
+        v3 += ldw(&cell_sq[k + 3 * st]);
     }
-    for (; k < b1; k += st) v0 += cell_sq[k];
-    return block_sum((v0 + v1) + (v2 + v3), sh);
+    for (; k < e; k += st) v0 += ldw(&cell_sq[k]);
+    const double t = block_sum((v0 + v1) + (v2 + v3), sh);
+    if (threadIdx.x < CASE_CTAS) {
+        // thread 0's sum into slot `rank` of every block of the cluster
+        const double mine = __shfl_sync((1u << CASE_CTAS) - 1u, t, 0);
+        *cl.map_shared_rank(&parts[rank], (int)threadIdx.x) = mine;
+    }
+    cl.sync();
+    double total = 0;
+    if (threadIdx.x == 0)
+        for (int r = 0; r < CASE_CTAS; ++r) total += parts[r];
+    return total;
 }
 
-static __global__ void __launch_bounds__(1024) k_case_control(const double* __restrict__ cell_sq,
-                                                             const int* __restrict__ case_off, CaseCtrl* cctrl,
-                                                             int* case_done, double* chist, Ctrl* ctrl, int n_cases,
-                                                             int uniform) {
-    __shared__ double sh[32];
-    if (!uniform && ctrl->done) return;
-    const int c = blockIdx.x;
+// Per-case norm and run_solver control of a batch (multigrid.h:195-234 for
+// every case): one cluster per case.  A case that stops is marked in case_done
+// (its cells then hold their state); the whole run stops when every case has.
+static __global__ void __cluster_dims__(CASE_CTAS, 1, 1) __launch_bounds__(CASE_THREADS)
+    k_case_control(const double* cell_sq, const int* __restrict__ case_off, CaseCtrl* cctrl, int* case_done,
+                   double* chist, Ctrl* ctrl, int n_cases, int uniform) {
+    __shared__ double sh[32], parts[CASE_CTAS];
+    pdl_wait();
+    const int c = blockIdx.x / CASE_CTAS;
     CaseCtrl& cc = cctrl[c];
-    if (!uniform && cc.done) return;
-    const int b0 = case_off[c], b1 = case_off[c + 1];
-    const double t = case_sum(cell_sq, b0, b1, sh);
-    if (threadIdx.x != 0) return;
+    if (!uniform && (ldw(&ctrl->done) || ldw(&cc.done))) return;  // the whole cluster alike
+    const double t = case_sum(cell_sq, __ldg(&case_off[c]), __ldg(&case_off[c + 1]), sh, parts);
+    if (blockIdx.x % CASE_CTAS != 0 || threadIdx.x != 0) return;
     const double norm = sqrt(t);
     if (uniform) {
         cc.err0 = norm;
@@ -1179,18 +1246,20 @@ static __global__ void __launch_bounds__(1024) k_case_control(const double* __re
 // Implicit batches, right after a right-hand side: a case whose face sums
 // are not finite stops (status 4) and its right-hand-side rows are zeroed
 // before the linear solve, so it cannot spread into the other cases.
-static __global__ void __launch_bounds__(1024) k_case_nonfinite(const double* __restrict__ cell_sq,
-                                                               const int* __restrict__ case_off, CaseCtrl* cctrl,
-                                                               int* case_done, Ctrl* ctrl, d4* __restrict__ b) {
-    __shared__ double sh[32];
+static __global__ void __cluster_dims__(CASE_CTAS, 1, 1) __launch_bounds__(CASE_THREADS)
+    k_case_nonfinite(const double* cell_sq, const int* __restrict__ case_off, CaseCtrl* cctrl, int* case_done,
+                     Ctrl* ctrl, d4* __restrict__ b) {
+    __shared__ double sh[32], parts[CASE_CTAS];
     __shared__ int bad;
-    const int c = blockIdx.x;
-    if (cctrl[c].done) return;
-    const int b0 = case_off[c], b1 = case_off[c + 1];
-    const double t = case_sum(cell_sq, b0, b1, sh);
+    pdl_wait();
+    const int c = blockIdx.x / CASE_CTAS, rank = blockIdx.x % CASE_CTAS;
+    if (ldw(&cctrl[c].done)) return;  // the whole cluster alike
+    const int b0 = __ldg(&case_off[c]), b1 = __ldg(&case_off[c + 1]);
+    const double t = case_sum(cell_sq, b0, b1, sh, parts);
+    cooperative_groups::this_cluster().sync();  // every block has read cctrl[c].done
     if (threadIdx.x == 0) {
         bad = !(t == t) || t > 1.7976931348623157e308;
-        if (bad) {
+        if (bad && rank == 0) {
             cctrl[c].status = 4;
             cctrl[c].done = 1;
             case_done[c] = 1;
@@ -1200,7 +1269,7 @@ static __global__ void __launch_bounds__(1024) k_case_nonfinite(const double* __
     __syncthreads();
     if (bad) {
         const double z[4] = {0, 0, 0, 0};
-        for (int k = b0 + threadIdx.x; k < b1; k += blockDim.x) st4(&b[k], z);
+        for (int k = b0 + rank * blockDim.x + threadIdx.x; k < b1; k += CASE_CTAS * blockDim.x) st4(&b[k], z);
     }
 }
 
@@ -1208,7 +1277,8 @@ static __global__ void __launch_bounds__(1024) k_case_nonfinite(const double* __
 // case has stopped (a separate launch, so no block of k_case_control sees
 // the run's flag change under it).
 static __global__ void k_batch_finalize(Ctrl* ctrl, int n_cases) {
-    if (ctrl->done) return;
+    pdl_wait();
+    if (ldw(&ctrl->done)) return;
     ctrl->iter += 1;
     if (ctrl->ndone >= n_cases) ctrl->done = 1;
 }
@@ -1216,10 +1286,11 @@ static __global__ void k_batch_finalize(Ctrl* ctrl, int n_cases) {
 // Residual-norm finalisation and the run_solver control (multigrid.h:195-234)
 // in one block: fixed-order sum of the partials -> ‖qW‖₂, err/err_0,
 // convergence test, history every 10th iteration.
-static __global__ void __launch_bounds__(1024) k_control(const double* __restrict__ partials, int n, Ctrl* ctrl,
+static __global__ void __launch_bounds__(1024) k_control(const double* partials, int n, Ctrl* ctrl,
                                                          double* hist, double* norms, int uniform) {
     __shared__ double sh[32];
-    if (!uniform && ctrl->done) return;
+    pdl_wait();
+    if (!uniform && ldw(&ctrl->done)) return;
     // four independent accumulators per thread keep four loads in flight
     double v0 = 0, v1 = 0, v2 = 0, v3 = 0;
     const int st = blockDim.x;

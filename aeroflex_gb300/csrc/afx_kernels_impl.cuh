@@ -50,6 +50,10 @@ KM<T> make_km(const StepArgs& a) {
 
 inline int nblocks(int n, int b) { return (n + b - 1) / b; }
 
+// threads of k_control for n partial sums: four per thread, so that a small run
+// does not wait for the sums of idle warps
+inline int control_threads(int n) { return n >= 4096 ? 1024 : (n >= 512 ? 256 : 64); }
+
 inline void mark(const StepArgs& a, int id, cudaStream_t s) {
     if (a.prof) a.prof->mark(id, s);
 }
@@ -64,18 +68,18 @@ void launch_prep(const StepArgs& a, const KM<T>& m, const V4<S>* q, cudaStream_t
     // the face and tile variants form dt in their first stage (EIG/DT)
     if (a.variant != 0) {
         if (a.second)
-            k_prep<T, S, true, true, false><<<nb, a.block, 0, s>>>(m, q, gx, gy, ph, dt, a.ctrl);
+            launch_pdl_if(a.pdl, k_prep<T, S, true, true, false>, nb, a.block, 0, s, m, q, gx, gy, ph, dt, a.ctrl);
         else if (a.need_grad)
-            k_prep<T, S, true, false, false><<<nb, a.block, 0, s>>>(m, q, gx, gy, ph, dt, a.ctrl);
+            launch_pdl_if(a.pdl, k_prep<T, S, true, false, false>, nb, a.block, 0, s, m, q, gx, gy, ph, dt, a.ctrl);
         else
             return;
     } else {
         if (a.second)
-            k_prep<T, S, true, true, true><<<nb, a.block, 0, s>>>(m, q, gx, gy, ph, dt, a.ctrl);
+            launch_pdl_if(a.pdl, k_prep<T, S, true, true, true>, nb, a.block, 0, s, m, q, gx, gy, ph, dt, a.ctrl);
         else if (a.need_grad)
-            k_prep<T, S, true, false, true><<<nb, a.block, 0, s>>>(m, q, gx, gy, ph, dt, a.ctrl);
+            launch_pdl_if(a.pdl, k_prep<T, S, true, false, true>, nb, a.block, 0, s, m, q, gx, gy, ph, dt, a.ctrl);
         else
-            k_prep<T, S, false, false, true><<<nb, a.block, 0, s>>>(m, q, gx, gy, ph, dt, a.ctrl);
+            launch_pdl_if(a.pdl, k_prep<T, S, false, false, true>, nb, a.block, 0, s, m, q, gx, gy, ph, dt, a.ctrl);
     }
     mark(a, K_PREP, s);
 }
@@ -98,26 +102,36 @@ void launch_stage_v(const StepArgs& a, const KM<T>& m, const V4<S>* qk, const V4
             if (smem > 48 * 1024)
                 cudaFuncSetAttribute(k_resid_tile<T, S, VISC, SECOND, true>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            k_resid_tile<T, S, VISC, SECOND, true><<<nb, a.block, smem, s>>>(m, tv, qk, qmem, gx, gy, ph, o, a.ctrl);
+            launch_pdl_if(a.pdl, k_resid_tile<T, S, VISC, SECOND, true>, nb, a.block, smem, s, m, tv, qk, qmem, gx,
+                          gy, ph, o,
+                       a.ctrl);
         } else {
             if (smem > 48 * 1024)
                 cudaFuncSetAttribute(k_resid_tile<T, S, VISC, SECOND, false>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            k_resid_tile<T, S, VISC, SECOND, false><<<nb, a.block, smem, s>>>(m, tv, qk, qmem, gx, gy, ph, o, a.ctrl);
+            launch_pdl_if(a.pdl, k_resid_tile<T, S, VISC, SECOND, false>, nb, a.block, smem, s, m, tv, qk, qmem, gx,
+                          gy, ph, o,
+                       a.ctrl);
         }
         mark(a, K_RESID_TILE, s);
     } else if (a.variant == 1) {
         const int nbf = nblocks(a.n_faces, a.block);
         if (first) {
-            k_face_flux<T, S, VISC, SECOND, true><<<nbf, a.block, 0, s>>>(
-                m, a.n_faces, qk, qmem, gx, gy, ph, (V4<T>*)a.fflux, (T*)a.feL, a.ctrl);
+            launch_pdl_if(a.pdl, k_face_flux<T, S, VISC, SECOND, true>, nbf, a.block, 0, s, m, a.n_faces, qk, qmem,
+                          gx, gy, ph,
+                       (V4<T>*)a.fflux, (T*)a.feL, a.ctrl);
             mark(a, K_FACE_FLUX, s);
-            k_cell_sum<T, S, true><<<nb, a.block, 0, s>>>(m, (const V4<T>*)a.fflux, (const T*)a.feL, o, a.ctrl);
+            launch_pdl_if(a.pdl, k_cell_sum<T, S, true>, nb, a.block, 0, s, m, (const V4<T>*)a.fflux,
+                          (const T*)a.feL, o,
+                       a.ctrl);
         } else {
-            k_face_flux<T, S, VISC, SECOND, false><<<nbf, a.block, 0, s>>>(
-                m, a.n_faces, qk, qmem, gx, gy, ph, (V4<T>*)a.fflux, (T*)a.feL, a.ctrl);
+            launch_pdl_if(a.pdl, k_face_flux<T, S, VISC, SECOND, false>, nbf, a.block, 0, s, m, a.n_faces, qk, qmem,
+                          gx, gy, ph,
+                       (V4<T>*)a.fflux, (T*)a.feL, a.ctrl);
             mark(a, K_FACE_FLUX, s);
-            k_cell_sum<T, S, false><<<nb, a.block, 0, s>>>(m, (const V4<T>*)a.fflux, (const T*)a.feL, o, a.ctrl);
+            launch_pdl_if(a.pdl, k_cell_sum<T, S, false>, nb, a.block, 0, s, m, (const V4<T>*)a.fflux,
+                          (const T*)a.feL, o,
+                       a.ctrl);
         }
         mark(a, K_CELL_SUM, s);
     } else {
@@ -202,7 +216,14 @@ StageOut<T, S> base_out(const StepArgs& a, int p) {
 // from q; three stages alpha = 1/4, 1/2, 1 with the limiter re-formed from
 // each stage state; the new state goes to parity p^1.
 template <class T, class S, bool SHADOW>
-void iteration(const StepArgs& a, int p, cudaStream_t s) {
+void iteration(const StepArgs& a0, int p, cudaStream_t s) {
+    // Iterations run from a graph, which already keeps the gaps between kernels
+    // short: programmatic dependents gain 3% at 4.19M cells and cost 9% at 17k
+    // (blocks of the next kernel take their places while the last ones of this
+    // kernel still run).  Evaluations launched one by one (residual, rhs) gain
+    // at every size.
+    StepArgs a = a0;
+    a.pdl = a.n_cells >= 500000;
     const KM<T> m = make_km<T>(a);
     const V4<S>* q = (const V4<S>*)a.qsh[p];
     launch_prep<T, S>(a, m, q, s);
@@ -213,11 +234,11 @@ void iteration(const StepArgs& a, int p, cudaStream_t s) {
         if (st > 0 && a.second) {
             const int nl = nblocks(a.n_cells, a.block);
             if constexpr (sizeof(T) == 4)
-                k_limiter_f32<S><<<nl, a.block, 0, s>>>(m, qk, (const V4<T>*)a.gx, (const V4<T>*)a.gy, (V4<T>*)a.phi,
-                                                        a.ctrl);
+                launch_pdl_if(a.pdl, k_limiter_f32<S>, nl, a.block, 0, s, m, qk, (const V4<T>*)a.gx, (const V4<T>*)a.gy,
+                           (V4<T>*)a.phi, a.ctrl);
             else
-                k_limiter<T, S><<<nl, a.block, 0, s>>>(m, qk, (const V4<T>*)a.gx, (const V4<T>*)a.gy, (V4<T>*)a.phi,
-                                                       a.ctrl);
+                launch_pdl_if(a.pdl, k_limiter<T, S>, nl, a.block, 0, s, m, qk, (const V4<T>*)a.gx, (const V4<T>*)a.gy,
+                           (V4<T>*)a.phi, a.ctrl);
             mark(a, K_LIMITER, s);
         }
         // Spalart-Allmaras: eddy viscosity of the stage state first
@@ -240,11 +261,13 @@ void iteration(const StepArgs& a, int p, cudaStream_t s) {
             sa_stage<T, S>(a, m, qk, a.sa_nu[p], nuk, st < 2 ? a.sa_nus[st] : a.sa_nu[p ^ 1], alpha[st], s);
     }
     if (a.n_cases > 0) {
-        k_case_control<<<a.n_cases, 1024, 0, s>>>(a.cell_sq, a.case_off, a.cctrl, a.case_done, a.chist, a.ctrl,
-                                                 a.n_cases, 0);
-        k_batch_finalize<<<1, 1, 0, s>>>(a.ctrl, a.n_cases);
+        launch_pdl_if(a.pdl, k_case_control, CASE_CTAS * a.n_cases, CASE_THREADS, 0, s, a.cell_sq, a.case_off,
+                      a.cctrl, a.case_done, a.chist,
+                   a.ctrl, a.n_cases, 0);
+        launch_pdl_if(a.pdl, k_batch_finalize, 1, 1, 0, s, a.ctrl, a.n_cases);
     } else {
-        k_control<<<1, 1024, 0, s>>>(a.partials, nblocks(a.n_cells, a.block), a.ctrl, a.hist, a.norms, 0);
+        launch_pdl_if(a.pdl, k_control, 1, control_threads(nblocks(a.n_cells, a.block)), 0, s, a.partials,
+                      nblocks(a.n_cells, a.block), a.ctrl, a.hist, a.norms, 0);
     }
     mark(a, K_CONTROL, s);
 }
@@ -305,10 +328,11 @@ void uniform(const StepArgs& a, int p, const double* qf, cudaStream_t s) {
                                                    qf[2], qf[3], (d4*)a.Rq, a.partials, a.qfar_case, a.case_of,
                                                    a.cell_sq);
     if (a.n_cases > 0)
-        k_case_control<<<a.n_cases, 1024, 0, s>>>(a.cell_sq, a.case_off, a.cctrl, a.case_done, a.chist, a.ctrl,
-                                                 a.n_cases, 1);
+        launch_pdl_if(a.pdl, k_case_control, CASE_CTAS * a.n_cases, CASE_THREADS, 0, s, a.cell_sq, a.case_off,
+                      a.cctrl, a.case_done, a.chist,
+                   a.ctrl, a.n_cases, 1);
     else
-        k_control<<<1, 1024, 0, s>>>(a.partials, nb, a.ctrl, a.hist, nullptr, 1);
+        launch_pdl_if(a.pdl, k_control, 1, control_threads(nb), 0, s, a.partials, nb, a.ctrl, a.hist, nullptr, 1);
 }
 
 // Implicit solver, Spalart-Allmaras: `sweeps` point-implicit nu~ updates

@@ -129,6 +129,7 @@ struct StepArgs {
     double cp = 1., Pr_L = 0.72, Pr_T = 0.9;
     double sa_nu_far = 0.;                 // nu~ of the far field, 3 mu_L / rho_inf
     Prof* prof = nullptr;      // eager profiling only (never inside a graph)
+    bool pdl = true;           // launch as programmatic dependents (afx_pdl.cuh)
 };
 
 // One explicit iteration reading parity p, writing parity p^1.

@@ -52,9 +52,10 @@ __device__ __forceinline__ int ldw(const int* p) {
 
 }  // namespace dev
 
+// on = false: an ordinary launch
 template <class... P, class... A>
-inline cudaError_t launch_pdl(void (*kernel)(P...), const dim3 grid, const dim3 block, const size_t smem,
-                              const cudaStream_t s, A... args) {
+inline cudaError_t launch_pdl_if(const bool on, void (*kernel)(P...), const dim3 grid, const dim3 block,
+                                 const size_t smem, const cudaStream_t s, A... args) {
     cudaLaunchConfig_t c = {};
     c.gridDim = grid;
     c.blockDim = block;
@@ -64,8 +65,14 @@ inline cudaError_t launch_pdl(void (*kernel)(P...), const dim3 grid, const dim3 
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     c.attrs = at;
-    c.numAttrs = 1;
+    c.numAttrs = on ? 1 : 0;
     return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
+template <class... P, class... A>
+inline cudaError_t launch_pdl(void (*kernel)(P...), const dim3 grid, const dim3 block, const size_t smem,
+                              const cudaStream_t s, A... args) {
+    return launch_pdl_if(true, kernel, grid, block, smem, s, args...);
 }
 
 }  // namespace afx
