@@ -119,6 +119,10 @@ __device__ __forceinline__ float dabs(float x) { return fabsf(x); }
 // goes into (a - b and a + (-b) are the same number; two branches of a sum are
 // formed one after the other in a warp whose lanes differ)
 __device__ __forceinline__ float flip(const float x, const bool neg) { return neg ? -x : x; }
+// a product on the integer lanes, in FP64 (fp64::mul)
+__device__ __forceinline__ float imul(const float a, const float b) { return a * b; }
+__device__ __forceinline__ double imul(const double a, const double b) { return fp64::mul(a, b); }
+template <class T> __device__ __forceinline__ T imul(const T a, const T b) { return a * b; }
 __device__ __forceinline__ double flip(const double x, const bool neg) {
     return fp64::of_bits(fp64::bits_of(x) ^ (neg ? 0x8000000000000000ull : 0ull));
 }
@@ -213,9 +217,12 @@ __device__ __forceinline__ void roe_flux(const T gamma, const T nx, const T ny, 
 // an exact factor): every quotient, root and compare in integer arithmetic
 // with shared denominators, and every factor of two folded into a sum as an
 // exact product or into a denominator's exponent, so each result has the bits
-// of the expression above.  What is left on the FP64 pipe are about 135 sums
-// and products; the compiler's form held it for 18 divisions at 7 and 6
-// roots at 7.6 instructions each beside 180 sums and products.
+// of the expression above.  What would be left on the FP64 pipe are about 135
+// sums and products (the compiler's form held it for 18 divisions at 7 and 6
+// roots at 7.6 instructions each beside 180 sums and products); 31 of the
+// products, and 16 of the reconstruction's, are given to the integer lanes,
+// which the quotients alone leave idle half of the time: k_face_flux on 1.57M
+// faces 1203 us at first, 630 without the compiler's divisions, 467 so.
 __device__ __forceinline__ double entropy_corr64(const double l, const double d, const fp64::Den& d2) {
     return fp64::less(d, l) ? l : fp64::quot(l * l + d * d, d2);
 }
@@ -253,14 +260,15 @@ __device__ __forceinline__ void roe_flux2(const double gamma, const double nx, c
     const double kF234_1 = lambda_c * rho;
     const double kF5 = quot(lambda_cp * (dp + rcV), cc2);
     const double cnx = c * nx, cny = c * ny, cV = c * V;
-    f[0] = (V_L * qL[0] + V_R * qR[0]) - (kF1 + kF234_0 + kF5);
-    f[1] = (V_L * qL[1] + pL * nx + V_R * qR[1] + pR * nx) -
-           (kF1 * (u - cnx) + kF234_0 * u + kF234_1 * (uR - uL - dV * nx) + kF5 * (u + cnx));
-    f[2] = (V_L * qL[2] + pL * ny + V_R * qR[2] + pR * ny) -
-           (kF1 * (v - cny) + kF234_0 * v + kF234_1 * (vR - vL - dV * ny) + kF5 * (v + cny));
-    f[3] = (V_L * (qL[3] + pL) + V_R * (qR[3] + pR)) -
-           (__fma_rn(0.5, kF234_0 * q2, kF1 * (h - cV)) + kF234_1 * (u * (uR - uL) + v * (vR - vL) - V * dV) +
-            kF5 * (h + cV));
+    // the products of these sums on the integer lanes, beside the FP64 pipe
+    f[0] = (mul(V_L, qL[0]) + mul(V_R, qR[0])) - (kF1 + kF234_0 + kF5);
+    f[1] = (mul(V_L, qL[1]) + mul(pL, nx) + mul(V_R, qR[1]) + mul(pR, nx)) -
+           (mul(kF1, u - cnx) + mul(kF234_0, u) + mul(kF234_1, uR - uL - mul(dV, nx)) + mul(kF5, u + cnx));
+    f[2] = (mul(V_L, qL[2]) + mul(pL, ny) + mul(V_R, qR[2]) + mul(pR, ny)) -
+           (mul(kF1, v - cny) + mul(kF234_0, v) + mul(kF234_1, vR - vL - mul(dV, ny)) + mul(kF5, v + cny));
+    f[3] = (mul(V_L, qL[3] + pL) + mul(V_R, qR[3] + pR)) -
+           (__fma_rn(0.5, mul(kF234_0, q2), mul(kF1, h - cV)) +
+            mul(kF234_1, mul(u, uR - uL) + mul(v, vR - vL) - mul(V, dV)) + mul(kF5, h + cV));
 }
 __device__ __forceinline__ void roe_flux(const double gamma, const double nx, const double ny, const double* qL,
                                          const double* qR, double* f) {
@@ -278,31 +286,32 @@ __device__ __forceinline__ void laminar_flux(const T gamma, const T Rgas, const 
     for (int k = 0; k < 4; ++k) qc[k] = T(0.5) * (qL[k] + qR[k]);
     const Div<T> i1(qc[0]), i2(qc[0] * qc[0]), i3(T(3));
     const T p = (gamma - T(1)) * (qc[3] - i1(T(0.5)) * (qc[1] * qc[1] + qc[2] * qc[2]));
+    // (FP64: half of the products on the integer lanes, as in roe_flux2)
     T gp0 = T(2) * gx[3];
-    gp0 -= i1(gx[1] * qc[1]) + i2(qc[1] * (gx[1] * qc[0] - gx[0] * qc[1]));
-    gp0 -= i1(gx[2] * qc[2]) + i2(qc[2] * (gx[2] * qc[0] - gx[0] * qc[2]));
+    gp0 -= i1(imul(gx[1], qc[1])) + i2(imul(qc[1], imul(gx[1], qc[0]) - gx[0] * qc[1]));
+    gp0 -= i1(imul(gx[2], qc[2])) + i2(imul(qc[2], imul(gx[2], qc[0]) - gx[0] * qc[2]));
     gp0 *= T(0.5) * (gamma - T(1));
     T gp1 = T(2) * gy[3];
-    gp1 -= i1(gy[1] * qc[1]) + i2(qc[1] * (gy[1] * qc[0] - gy[0] * qc[1]));
-    gp1 -= i1(gy[2] * qc[2]) + i2(qc[2] * (gy[2] * qc[0] - gy[0] * qc[2]));
+    gp1 -= i1(imul(gy[1], qc[1])) + i2(imul(qc[1], imul(gy[1], qc[0]) - gy[0] * qc[1]));
+    gp1 -= i1(imul(gy[2], qc[2])) + i2(imul(qc[2], imul(gy[2], qc[0]) - gy[0] * qc[2]));
     gp1 *= T(0.5) * (gamma - T(1));
     const T Rinv = fdiv(T(1), Rgas);
-    const T gT0 = Rinv * i2(gp0 * qc[0] - gx[0] * p);
-    const T gT1 = Rinv * i2(gp1 * qc[0] - gy[0] * p);
-    const T gu0 = i2(qc[0] * gx[1] - qc[1] * gx[0]);
-    const T gu1 = i2(qc[0] * gy[1] - qc[1] * gy[0]);
-    const T gv0 = i2(qc[0] * gx[2] - qc[2] * gx[0]);
-    const T gv1 = i2(qc[0] * gy[2] - qc[2] * gy[0]);
+    const T gT0 = Rinv * i2(imul(gp0, qc[0]) - gx[0] * p);
+    const T gT1 = Rinv * i2(imul(gp1, qc[0]) - gy[0] * p);
+    const T gu0 = i2(imul(qc[0], gx[1]) - qc[1] * gx[0]);
+    const T gu1 = i2(imul(qc[0], gy[1]) - qc[1] * gy[0]);
+    const T gv0 = i2(imul(qc[0], gx[2]) - qc[2] * gx[0]);
+    const T gv1 = i2(imul(qc[0], gy[2]) - qc[2] * gy[0]);
     const T div3 = i3(gu0 + gv1);
     const T tau_xx = T(2) * mu * (gu0 - div3);
     const T tau_yy = T(2) * mu * (gv1 - div3);
     const T tau_xy = mu * (gu1 + gv0);
     const T uc = i1(qc[1]), vc = i1(qc[2]);
-    const T phi0 = uc * tau_xx + vc * tau_xy + kheat * gT0;
-    const T phi1 = uc * tau_xy + vc * tau_yy + kheat * gT1;
-    f[1] -= nx * tau_xx + ny * tau_xy;
-    f[2] -= nx * tau_xy + ny * tau_yy;
-    f[3] -= nx * phi0 + ny * phi1;
+    const T phi0 = imul(uc, tau_xx) + vc * tau_xy + kheat * gT0;
+    const T phi1 = imul(uc, tau_xy) + vc * tau_yy + kheat * gT1;
+    f[1] -= imul(nx, tau_xx) + ny * tau_xy;
+    f[2] -= imul(nx, tau_xy) + ny * tau_yy;
+    f[3] -= imul(nx, phi0) + ny * phi1;
 }
 
 // Boundary ghost state from the interior state qL and the stored boundary

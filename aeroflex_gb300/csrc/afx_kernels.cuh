@@ -460,6 +460,13 @@ __device__ __forceinline__ void reconstruct(const T* q, const T* gxc, const T* g
     for (int k = 0; k < 4; ++k) out[k] = q[k] + (gxc[k] * dx + gyc[k] * dy) * ph[k];
 }
 
+// (FP64: two of its three products on the integer lanes)
+__device__ __forceinline__ void reconstruct(const double* q, const double* gxc, const double* gyc, const double* ph,
+                                            const double dx, const double dy, double* out) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) out[k] = q[k] + fp64::mul(gxc[k] * dx + fp64::mul(gyc[k], dy), ph[k]);
+}
+
 // average_gradients (solver.h:359-398) for the laminar face flux: member
 // states qa/qb and gradients of the face's two cells, direction from the
 // precomputed sum-of-centroids vector t = (t0, t1, lij).

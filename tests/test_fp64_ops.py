@@ -1,5 +1,5 @@
-"""Integer FP64 division, square root and ordering (csrc/afx_fp64.cuh) against
-the host's IEEE operations: bit for bit, with the reciprocal seeds off by up
+"""Integer FP64 division, square root, product, conversions and ordering
+(csrc/afx_fp64.cuh) against the host's IEEE operations: bit for bit, with the reciprocal seeds off by up
 to 3 units in their last place either way."""
 import os
 import subprocess
@@ -39,6 +39,11 @@ int main(int argc, char** argv) {
         const Den d = den(y);
         bad += !same(quot(x, d), x / y) || !same(quot(x, twice(d)), x / (2.0 * y));
         bad += !same(root(std::fabs(x)), std::sqrt(std::fabs(x))) || !same(root(x), std::sqrt(x));
+        bad += !same(mul(x, y), x * y);
+        uint32_t r;
+        if (narrow(x, r)) bad += f32_bits((float)x) != r;
+        const float xf = (float)x;
+        if (std::fabs(xf) >= 1.17549435e-38f || xf == 0.f || xf != xf) bad += !same(widen(f32_bits(xf)), (double)xf);
         bad += less(x, y) != (x < y) || less_equal(x, y) != (x <= y) || less_equal(x, x) != (x <= x);
         const double s = y * y;  // next to exact squares
         if (s > 1e-300 && s < 1e300)
