@@ -119,9 +119,14 @@ __device__ __forceinline__ float dabs(float x) { return fabsf(x); }
 // goes into (a - b and a + (-b) are the same number; two branches of a sum are
 // formed one after the other in a warp whose lanes differ)
 __device__ __forceinline__ float flip(const float x, const bool neg) { return neg ? -x : x; }
-// a product on the integer lanes, in FP64 (fp64::mul)
-__device__ __forceinline__ float imul(const float a, const float b) { return a * b; }
+// a product on the integer lanes, in FP64 (fp64::mul); a unit compiled with
+// contraction keeps it on the FP64 pipe, where most products go into a fused
+// multiply-add with the sum that follows
+#ifdef AFX_CONTRACTED
+__device__ __forceinline__ double imul(const double a, const double b) { return a * b; }
+#else
 __device__ __forceinline__ double imul(const double a, const double b) { return fp64::mul(a, b); }
+#endif
 template <class T> __device__ __forceinline__ T imul(const T a, const T b) { return a * b; }
 __device__ __forceinline__ double flip(const double x, const bool neg) {
     return fp64::of_bits(fp64::bits_of(x) ^ (neg ? 0x8000000000000000ull : 0ull));
@@ -261,14 +266,14 @@ __device__ __forceinline__ void roe_flux2(const double gamma, const double nx, c
     const double kF5 = quot(lambda_cp * (dp + rcV), cc2);
     const double cnx = c * nx, cny = c * ny, cV = c * V;
     // the products of these sums on the integer lanes, beside the FP64 pipe
-    f[0] = (mul(V_L, qL[0]) + mul(V_R, qR[0])) - (kF1 + kF234_0 + kF5);
-    f[1] = (mul(V_L, qL[1]) + mul(pL, nx) + mul(V_R, qR[1]) + mul(pR, nx)) -
-           (mul(kF1, u - cnx) + mul(kF234_0, u) + mul(kF234_1, uR - uL - mul(dV, nx)) + mul(kF5, u + cnx));
-    f[2] = (mul(V_L, qL[2]) + mul(pL, ny) + mul(V_R, qR[2]) + mul(pR, ny)) -
-           (mul(kF1, v - cny) + mul(kF234_0, v) + mul(kF234_1, vR - vL - mul(dV, ny)) + mul(kF5, v + cny));
-    f[3] = (mul(V_L, qL[3] + pL) + mul(V_R, qR[3] + pR)) -
-           (__fma_rn(0.5, mul(kF234_0, q2), mul(kF1, h - cV)) +
-            mul(kF234_1, mul(u, uR - uL) + mul(v, vR - vL) - mul(V, dV)) + mul(kF5, h + cV));
+    f[0] = (imul(V_L, qL[0]) + imul(V_R, qR[0])) - (kF1 + kF234_0 + kF5);
+    f[1] = (imul(V_L, qL[1]) + imul(pL, nx) + imul(V_R, qR[1]) + imul(pR, nx)) -
+           (imul(kF1, u - cnx) + imul(kF234_0, u) + imul(kF234_1, uR - uL - imul(dV, nx)) + imul(kF5, u + cnx));
+    f[2] = (imul(V_L, qL[2]) + imul(pL, ny) + imul(V_R, qR[2]) + imul(pR, ny)) -
+           (imul(kF1, v - cny) + imul(kF234_0, v) + imul(kF234_1, vR - vL - imul(dV, ny)) + imul(kF5, v + cny));
+    f[3] = (imul(V_L, qL[3] + pL) + imul(V_R, qR[3] + pR)) -
+           (__fma_rn(0.5, imul(kF234_0, q2), imul(kF1, h - cV)) +
+            imul(kF234_1, imul(u, uR - uL) + imul(v, vR - vL) - imul(V, dV)) + imul(kF5, h + cV));
 }
 __device__ __forceinline__ void roe_flux(const double gamma, const double nx, const double ny, const double* qL,
                                          const double* qR, double* f) {

@@ -35,6 +35,7 @@
 #include <string>
 #include <vector>
 
+#define AFX_CONTRACTED  // this unit is compiled with multiply-add contraction
 #include "afx_host.hpp"
 #include "afx_kernels_impl.cuh"
 #include "afx_pdl.cuh"

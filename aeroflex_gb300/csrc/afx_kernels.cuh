@@ -464,7 +464,7 @@ __device__ __forceinline__ void reconstruct(const T* q, const T* gxc, const T* g
 __device__ __forceinline__ void reconstruct(const double* q, const double* gxc, const double* gyc, const double* ph,
                                             const double dx, const double dy, double* out) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) out[k] = q[k] + fp64::mul(gxc[k] * dx + fp64::mul(gyc[k], dy), ph[k]);
+    for (int k = 0; k < 4; ++k) out[k] = q[k] + imul(gxc[k] * dx + imul(gyc[k], dy), ph[k]);
 }
 
 // average_gradients (solver.h:359-398) for the laminar face flux: member

@@ -54,7 +54,7 @@ __device__ __forceinline__ T sa_cbrt(T x) {
     mm = sa_ldexp(mm, r);
     T y = T(0.7) + T(0.3) * mm;
 #pragma unroll 1
-    for (int it = 0; it < 7; ++it) y = y - (y * y * y - mm) / (T(3) * y * y);
+    for (int it = 0; it < 7; ++it) y = y - fdiv(y * y * y - mm, T(3) * y * y);
     return sa_ldexp(y, e3);
 }
 
@@ -62,23 +62,26 @@ __device__ __forceinline__ T sa_cbrt(T x) {
 template <class T>
 __device__ __forceinline__ void sa_source(const T nut, const T nul, const T omega, const T d, T* src, T* dsrc) {
     const T d2 = d * d;
+    const Div<T> id2(d2);
     if (nut < T(0)) {
         const T P = T(SA_CB1) * (T(1) - T(SA_CT3)) * omega * nut;
-        const T D = -T(SA_CW1) * (nut * nut) / d2;
+        const T D = id2(-T(SA_CW1) * (nut * nut));
         *src = P - D;
-        *dsrc = T(SA_CB1) * (T(1) - T(SA_CT3)) * omega + T(2) * T(SA_CW1) * nut / d2;
+        *dsrc = T(SA_CB1) * (T(1) - T(SA_CT3)) * omega + id2(T(2) * T(SA_CW1) * nut);
         return;
     }
     const T cv13 = T(SA_CV1) * T(SA_CV1) * T(SA_CV1);
-    const T chi = nut / nul;
+    const Div<T> inul(nul);
+    const T chi = inul(nut);
     const T chi3 = chi * chi * chi;
-    const T fv1 = chi3 / (chi3 + cv13);
-    const T dfv1 = T(3) * chi * chi * cv13 / ((chi3 + cv13) * (chi3 + cv13)) / nul;
-    const T fv2 = T(1) - chi / (T(1) + chi * fv1);
-    const T dfv2 = -(T(1) / nul - chi * chi * dfv1) / ((T(1) + chi * fv1) * (T(1) + chi * fv1));
+    const T fv1 = fdiv(chi3, chi3 + cv13);
+    const T dfv1 = inul(fdiv(T(3) * chi * chi * cv13, (chi3 + cv13) * (chi3 + cv13)));
+    const T fv2 = T(1) - fdiv(chi, T(1) + chi * fv1);
+    const T dfv2 = fdiv(-(inul(T(1)) - chi * chi * dfv1), (T(1) + chi * fv1) * (T(1) + chi * fv1));
     const T kd2 = T(SA_KAPPA) * T(SA_KAPPA) * d2;
-    const T Sbar = nut * fv2 / kd2;
-    const T dSbar = (fv2 + nut * dfv2) / kd2;
+    const Div<T> ikd2(kd2);
+    const T Sbar = ikd2(nut * fv2);
+    const T dSbar = ikd2(fv2 + nut * dfv2);
     T Stil, dStil;
     if (Sbar >= -T(SA_CV2) * omega) {
         Stil = omega + Sbar;
@@ -86,15 +89,15 @@ __device__ __forceinline__ void sa_source(const T nut, const T nul, const T omeg
     } else {
         const T num = T(SA_CV2) * T(SA_CV2) * omega + T(SA_CV3) * Sbar;
         const T den = (T(SA_CV3) - T(2) * T(SA_CV2)) * omega - Sbar;
-        Stil = omega + omega * num / den;
-        dStil = omega * dSbar * (T(SA_CV3) * den + num) / (den * den);
+        Stil = omega + fdiv(omega * num, den);
+        dStil = fdiv(omega * dSbar * (T(SA_CV3) * den + num), den * den);
     }
     T r = T(10), dr = T(0);
     if (Stil > T(0)) {
-        const T rr = nut / (Stil * kd2);
+        const T rr = fdiv(nut, Stil * kd2);
         if (rr < T(10)) {
             r = rr;
-            dr = (Stil - nut * dStil) / (Stil * Stil * kd2);
+            dr = fdiv(Stil - nut * dStil, Stil * Stil * kd2);
         }
     }
     const T r2 = r * r;
@@ -103,13 +106,14 @@ __device__ __forceinline__ void sa_source(const T nut, const T nul, const T omeg
     const T cw36 = T(SA_CW3) * T(SA_CW3) * T(SA_CW3) * T(SA_CW3) * T(SA_CW3) * T(SA_CW3);
     const T g2 = g * g;
     const T g6 = g2 * g2 * g2;
-    const T s6 = dsqrt(sa_cbrt((T(1) + cw36) / (g6 + cw36)));
+    const Div<T> ig(g6 + cw36);
+    const T s6 = dsqrt(sa_cbrt(ig(T(1) + cw36)));
     const T fw = g * s6;
-    const T dfw = s6 * cw36 / (g6 + cw36) * dg;
+    const T dfw = ig(s6 * cw36) * dg;
     const T P = T(SA_CB1) * Stil * nut;
-    const T D = T(SA_CW1) * fw * (nut * nut) / d2;
+    const T D = id2(T(SA_CW1) * fw * (nut * nut));
     *src = P - D;
-    *dsrc = T(SA_CB1) * (dStil * nut + Stil) - T(SA_CW1) * (dfw * (nut * nut) + fw * T(2) * nut) / d2;
+    *dsrc = T(SA_CB1) * (dStil * nut + Stil) - id2(T(SA_CW1) * (dfw * (nut * nut) + fw * T(2) * nut));
 }
 
 // The pointers of one SA evaluation (device cell order).
@@ -142,9 +146,9 @@ __global__ void __launch_bounds__(256) k_sa_mut(const int n, const V4<S>* __rest
     T out = T(0);
     if (nt >= T(0)) {
         const T cv13 = T(SA_CV1) * T(SA_CV1) * T(SA_CV1);
-        const T chi = nt * rho / mu;
+        const T chi = fdiv(nt * rho, mu);
         const T chi3 = chi * chi * chi;
-        out = rho * nt * (chi3 / (chi3 + cv13));
+        out = rho * nt * fdiv(chi3, chi3 + cv13);
     }
     mut[i] = out;
 }
@@ -160,15 +164,17 @@ __device__ __forceinline__ T sa_cell_residual(const KM<T>& m, const V4<S>* __res
     ld4c<T>(&gx[i], gxi);
     ld4c<T>(&gy[i], gyi);
     const T rho_i = qi[0];
-    const T u_i = qi[1] / rho_i, v_i = qi[2] / rho_i;
-    const T nul_i = m.mu / rho_i;
+    const Div<T> ir(rho_i), ir2(rho_i * rho_i);
+    const T u_i = ir(qi[1]), v_i = ir(qi[2]);
+    const T nul_i = ir(m.mu);
     const T nut_i = (T)__ldg(&v.nuk[i]);
-    const T du_dy = (rho_i * gyi[1] - qi[1] * gyi[0]) / (rho_i * rho_i);
-    const T dv_dx = (rho_i * gxi[2] - qi[2] * gxi[0]) / (rho_i * rho_i);
+    const T du_dy = ir2(rho_i * gyi[1] - qi[1] * gyi[0]);
+    const T dv_dx = ir2(rho_i * gxi[2] - qi[2] * gxi[0]);
     const T omega = dabs(dv_dx - du_dy);
     const V2<T> ci = __ldg(&v.cxy[i]);
     const int4 sl = __ldg(&m.cslot[i]);
     const int4 nb = __ldg(&m.cnbr[i]);
+    const Div<T> isg((T(SA_SIGMA)));
     T conv = T(0), diff = T(0), ggx = T(0), ggy = T(0), couple = T(0);
 #pragma unroll 1
     for (int s = 0; s < 4; ++s) {
@@ -181,14 +187,14 @@ __device__ __forceinline__ T sa_cell_residual(const KM<T>& m, const V4<S>* __res
         const T nox = own0 ? n.x : -n.x;
         const T noy = own0 ? n.y : -n.y;
         const T L = __ldg(&m.fLg[f]).x;
-        T rho_j, u_j, v_j, nut_j;
+        T rho_j, ru_j, rv_j, nut_j;
         V2<T> cj;
         if (oc >= 0) {
             T qj[4];
             ld4s(&qk[oc], qj);
             rho_j = qj[0];
-            u_j = qj[1] / rho_j;
-            v_j = qj[2] / rho_j;
+            ru_j = qj[1];
+            rv_j = qj[2];
             nut_j = (T)__ldg(&v.nuk[oc]);
             cj = __ldg(&v.cxy[oc]);
         } else {
@@ -198,12 +204,14 @@ __device__ __forceinline__ T sa_cell_residual(const KM<T>& m, const V4<S>* __res
             ld4c<T>(&m.bq[b], qb);
             ghost_state(bt, m.gamma, n.x, n.y, qi, qb, qg);
             rho_j = qg[0];
-            u_j = qg[1] / qg[0];
-            v_j = qg[2] / qg[0];
+            ru_j = qg[1];
+            rv_j = qg[2];
             nut_j = bt == BT_WALL ? -nut_i : (bt == BT_FARFIELD ? v.nu_far : nut_i);
             cj = __ldg(&v.gxy[b]);
         }
-        const T nul_j = m.mu / rho_j;
+        const Div<T> irj(rho_j);
+        const T u_j = irj(ru_j), v_j = irj(rv_j);
+        const T nul_j = irj(m.mu);
         const T un = T(0.5) * (u_i + u_j) * nox + T(0.5) * (v_i + v_j) * noy;
         conv += L * smin(un, T(0)) * (nut_j - nut_i);
         const T dx = cj.x - ci.x;
@@ -214,22 +222,24 @@ __device__ __forceinline__ T sa_cell_residual(const KM<T>& m, const V4<S>* __res
         const T ntf = T(0.5) * (nut_i + nut_j);
         T fn = T(1);
         if (ntf < T(0)) {
-            const T chi = ntf / nuf;
+            const T chi = fdiv(ntf, nuf);
             const T chi3 = chi * chi * chi;
-            fn = (T(SA_CN1) + chi3) / (T(SA_CN1) - chi3);
+            fn = fdiv(T(SA_CN1) + chi3, T(SA_CN1) - chi3);
         }
-        diff += L * (nuf + fn * ntf) * (nut_j - nut_i) * ddn / dd;
+        const Div<T> idd(dd);
+        diff += idd(L * (nuf + fn * ntf) * (nut_j - nut_i) * ddn);
         ggx += ntf * nox * L;
         ggy += ntf * noy * L;
         if (DIAG)
-            couple += L * (-smin(un, T(0))) + L * smax(nuf + fn * ntf, T(0)) * smax(ddn, T(0)) / dd / T(SA_SIGMA);
+            couple += L * (-smin(un, T(0))) + isg(idd(L * smax(nuf + fn * ntf, T(0)) * smax(ddn, T(0))));
     }
     const T A = __ldg(&m.area[i]);
-    const T gnx = ggx / A, gny = ggy / A;
+    const Div<T> iA(A);
+    const T gnx = iA(ggx), gny = iA(ggy);
     T src, dsrc;
     sa_source(nut_i, nul_i, omega, __ldg(&v.wd[i]), &src, &dsrc);
-    if (DIAG) *diag = A / __ldg(&v.dt[i]) + couple + A * smax(-dsrc, T(0));
-    return -conv + diff / T(SA_SIGMA) + T(SA_CB2) / T(SA_SIGMA) * (gnx * gnx + gny * gny) * A + src * A;
+    if (DIAG) *diag = fdiv(A, __ldg(&v.dt[i])) + couple + A * smax(-dsrc, T(0));
+    return -conv + isg(diff) + T(SA_CB2) / T(SA_SIGMA) * (gnx * gnx + gny * gny) * A + src * A;
 }
 
 // One RK stage of nu~ (solver.h:802-828 applied to the SA equation): R / A
@@ -243,7 +253,7 @@ __global__ void __launch_bounds__(256) k_sa_stage(const KM<T> m, const V4<S>* __
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m.n_cells) return;
     const T R = sa_cell_residual<T, S, false>(m, qk, gx, gy, v, i, nullptr);
-    const T nuW = R / __ldg(&m.area[i]);
+    const T nuW = fdiv(R, __ldg(&m.area[i]));
     v.nuW[i] = (double)nuW;
     if (v.nu_next) {
         const T inc = nuW * __ldg(&v.dt[i]) * (T)v.alpha * (T)v.relax;
@@ -262,8 +272,8 @@ __global__ void __launch_bounds__(256) k_sa_implicit(const KM<T> m, const V4<S>*
     if (i >= m.n_cells) return;
     T diag = T(1);
     const T R = sa_cell_residual<T, S, true>(m, qk, gx, gy, v, i, &diag);
-    v.nuW[i] = (double)(R / __ldg(&m.area[i]));
-    v.nu_next[i] = __ldg(&v.nuk[i]) + (double)((T)v.relax * R / diag);
+    v.nuW[i] = (double)fdiv(R, __ldg(&m.area[i]));
+    v.nu_next[i] = __ldg(&v.nuk[i]) + (double)fdiv((T)v.relax * R, diag);
 }
 
 }  // namespace dev
