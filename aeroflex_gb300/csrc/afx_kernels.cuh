@@ -52,25 +52,18 @@ __device__ __forceinline__ void l2_ahead(const void* base, const int size, const
                      :: "l"(reinterpret_cast<const char*>(base) + b), "r"((unsigned)(e - b)));
 }
 
-// The cell's limiter (solver.h:517-593): per variable the least limiter_value
-// over its faces, at most 1.  sl: the cell's slots (0: none); dx, dy: face
-// centre minus centroid per slot.
+// The cell's limiter of one variable (solver.h:517-593): the least limiter_value
+// over its faces, at most 1.  slots: bit s for slot s in use; dx, dy: face centre
+// minus centroid per slot; dmx, dmn: the neighbours' extremes less the cell's
+// value.
 template <class T>
-__device__ __forceinline__ void cell_limiter(const KM<T>& m, const int4 sl, const T* qi, const T* qmn, const T* qmx,
-                                             const T* gx, const T* gy, const T* dx, const T* dy, const T K3a,
-                                             T* lim) {
+__device__ __forceinline__ T limiter_of(const int kind, const unsigned slots, const T dmx, const T dmn, const T gx,
+                                        const T gy, const T* dx, const T* dy, const T K3a) {
+    T lim = T(1);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) lim[k] = T(1);
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-        if (pick(sl, s) != 0) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const T dqg = gx[k] * dx[s] + gy[k] * dy[s];
-                lim[k] = smin(lim[k], limiter_value(m.limiter, dqg, qmx[k] - qi[k], qmn[k] - qi[k], K3a));
-            }
-        }
-    }
+    for (int s = 0; s < 4; ++s)
+        if (slots >> s & 1u) lim = smin(lim, limiter_value(kind, gx * dx[s] + gy * dy[s], dmx, dmn, K3a));
+    return lim;
 }
 
 // FP64: the least value over the faces is looked for in FP32 first, and only
@@ -92,55 +85,47 @@ __device__ __forceinline__ float f32_toward_zero(const double x) {
     const uint32_t mag = ((uint32_t)e << 23) | ((hi & 0xfffffu) << 3) | ((uint32_t)u >> 29);
     return __uint_as_float((e <= 0 ? 0u : (e >= 255 ? 0x7f800000u : mag)) | (hi & 0x80000000u));
 }
-template <>
-__device__ __forceinline__ void cell_limiter<double>(const KM<double>& m, const int4 sl, const double* qi,
-                                                     const double* qmn, const double* qmx, const double* gx,
-                                                     const double* gy, const double* dx, const double* dy,
-                                                     const double K3a, double* lim) {
-    float dxf[4], dyf[4];
-    unsigned slots = 0;
+__device__ __forceinline__ double limiter_of(const int kind, const unsigned slots, const double dmx, const double dmn,
+                                             const double gx, const double gy, const double* dx, const double* dy,
+                                             const double K3a) {
+    unsigned mask = slots;
+    if (kind == 0) {
+        const float Kf = f32_toward_zero(K3a), gxf = f32_toward_zero(gx), gyf = f32_toward_zero(gy);
+        const float up = f32_toward_zero(dmx), dn = -f32_toward_zero(dmn);
+        float lo[4], best = 0.f;
 #pragma unroll
-    for (int s = 0; s < 4; ++s) {
-        dxf[s] = f32_toward_zero(dx[s]);
-        dyf[s] = f32_toward_zero(dy[s]);
-        slots |= pick(sl, s) != 0 ? 1u << s : 0u;
-    }
-    const float Kf = f32_toward_zero(K3a);
-    const bool venk = m.limiter == 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const double dmx = qmx[k] - qi[k], dmn = qmn[k] - qi[k];
-        unsigned mask = slots;
-        if (venk) {
-            const float gxf = f32_toward_zero(gx[k]), gyf = f32_toward_zero(gy[k]);
-            const float up = f32_toward_zero(dmx), dn = -f32_toward_zero(dmn);
-            float lo[4], best = 0.f;
-#pragma unroll
-            for (int s = 0; s < 4; ++s) {
-                const float a = __fmul_rn(gxf, dxf[s]), b = __fmul_rn(gyf, dyf[s]), g = a + b;
-                const float ag = fabsf(g), err = 1e-6f * (fabsf(a) + fabsf(b)), D = g > 0.f ? up : dn;
-                const float Q = D * D + 2.f * ag * ag + D * ag + Kf, iQ = __fdividef(1.f, Q);
-                const float v = ag * (D - 2.f * ag) * iQ;
-                const float tol = (4e-6f * ag * (D + 2.f * ag) + err * (3.f * D + 12.f * ag)) * iQ + 1e-14f;
-                const bool plain = ag > err + 1.2e-16f && Q > 1e-30f && Q < 1e30f;
-                const bool off = ag + err < 0.8e-16f;  // below the threshold for certain: the value is 1
-                lo[s] = plain ? v - tol : (off ? 1.f : -1e30f);
-                if (plain && (slots >> s & 1u)) best = fminf(best, v + tol);
-            }
-#pragma unroll
-            for (int s = 0; s < 4; ++s)
-                if (lo[s] > best) mask &= ~(1u << s);
+        for (int s = 0; s < 4; ++s) {
+            const float a = __fmul_rn(gxf, f32_toward_zero(dx[s])), b = __fmul_rn(gyf, f32_toward_zero(dy[s]));
+            const float g = a + b, ag = fabsf(g), err = 1e-6f * (fabsf(a) + fabsf(b)), D = g > 0.f ? up : dn;
+            const float Q = D * D + 2.f * ag * ag + D * ag + Kf, iQ = __fdividef(1.f, Q);
+            const float v = ag * (D - 2.f * ag) * iQ;
+            const float tol = (4e-6f * ag * (D + 2.f * ag) + err * (3.f * D + 12.f * ag)) * iQ + 1e-14f;
+            const bool plain = ag > err + 1.2e-16f && Q > 1e-30f && Q < 1e30f;
+            const bool off = ag + err < 0.8e-16f;  // below the threshold for certain: the value is 1
+            lo[s] = plain ? v - tol : (off ? 1.f : -1e30f);
+            if (plain && (slots >> s & 1u)) best = fminf(best, v + tol);
         }
-        double l = 1.0;
-        while (mask) {
-            const int s = __ffs(mask) - 1;
-            mask &= mask - 1;
-            const double x = s == 0 ? dx[0] : s == 1 ? dx[1] : s == 2 ? dx[2] : dx[3];
-            const double y = s == 0 ? dy[0] : s == 1 ? dy[1] : s == 2 ? dy[2] : dy[3];
-            l = smin(l, limiter_value(m.limiter, gx[k] * x + gy[k] * y, dmx, dmn, K3a));
-        }
-        lim[k] = l;
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+            if (lo[s] > best) mask &= ~(1u << s);
     }
+    double l = 1.0;
+    while (mask) {
+        const int s = __ffs(mask) - 1;
+        mask &= mask - 1;
+        const double x = s == 0 ? dx[0] : s == 1 ? dx[1] : s == 2 ? dx[2] : dx[3];
+        const double y = s == 0 ? dy[0] : s == 1 ? dy[1] : s == 2 ? dy[2] : dy[3];
+        l = smin(l, limiter_value(kind, gx * x + gy * y, dmx, dmn, K3a));
+    }
+    return l;
+}
+template <class T>
+__device__ __forceinline__ T limiter_K3(const T limk, const T A) {
+    const T Ka = limk * dsqrt(A);
+    return Ka * Ka * Ka;
+}
+__device__ __forceinline__ unsigned slots_of(const int4 sl) {
+    return (sl.x != 0 ? 1u : 0u) | (sl.y != 0 ? 2u : 0u) | (sl.z != 0 ? 4u : 0u) | (sl.w != 0 ? 8u : 0u);
 }
 
 // Per cell, from the iteration's starting state q (the solver's member q):
@@ -299,11 +284,11 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_prep(const KM<T
     gx[i] = vx;
     gy[i] = vy;
     if (!SECOND) return;
-    const T sqrt_area = dsqrt(A);
-    const T Ka = m.limk * sqrt_area;
-    const T K3a = Ka * Ka * Ka;
+    const T K3a = limiter_K3(m.limk, A);
     T lim[4];
-    cell_limiter<T>(m, sl, qi, qmn, qmx, gxi, gyi, dxs, dys, K3a, lim);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        lim[k] = limiter_of(m.limiter, slots_of(sl), qmx[k] - qi[k], qmn[k] - qi[k], gxi[k], gyi[k], dxs, dys, K3a);
     V4<T> vp;
     st4(&vp, lim);
     phi[i] = vp;
@@ -364,11 +349,11 @@ __global__ void __launch_bounds__(256) k_limiter(const KM<T> m, const V4<S>* __r
             }
         }
     }
-    const T sqrt_area = dsqrt(A);
-    const T Ka = m.limk * sqrt_area;
-    const T K3a = Ka * Ka * Ka;
+    const T K3a = limiter_K3(m.limk, A);
     T lim[4];
-    cell_limiter<T>(m, sl, qi, qmn, qmx, gxi, gyi, dxs, dys, K3a, lim);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        lim[k] = limiter_of(m.limiter, slots_of(sl), qmx[k] - qi[k], qmn[k] - qi[k], gxi[k], gyi[k], dxs, dys, K3a);
     V4<T> vp;
     st4(&vp, lim);
     phi[i] = vp;
@@ -442,13 +427,155 @@ __global__ void __launch_bounds__(256) k_limiter_f32(const KM<float> m, const V4
             }
         }
     }
-    const float sqrt_area = dsqrt(A);
-    const float Ka = m.limk * sqrt_area;
-    const float K3a = Ka * Ka * Ka;
+    const float K3a = limiter_K3(m.limk, A);
     float lim[4];
-    const int4 on = make_int4(nb.x != NO_NEIGHBOUR, nb.y != NO_NEIGHBOUR, nb.z != NO_NEIGHBOUR, nb.w != NO_NEIGHBOUR);
-    cell_limiter<float>(m, on, qi, qmn, qmx, gxi, gyi, dxs, dys, K3a, lim);
+    const unsigned on = (nb.x != NO_NEIGHBOUR ? 1u : 0u) | (nb.y != NO_NEIGHBOUR ? 2u : 0u) |
+                        (nb.z != NO_NEIGHBOUR ? 4u : 0u) | (nb.w != NO_NEIGHBOUR ? 8u : 0u);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        lim[k] = limiter_of(m.limiter, on, qmx[k] - qi[k], qmn[k] - qi[k], gxi[k], gyi[k], dxs, dys, K3a);
     phi[i] = make_float4(lim[0], lim[1], lim[2], lim[3]);
+}
+
+// k_prep and k_limiter with four lanes per cell, one per variable: gradients
+// and limiters of the variables do not depend on one another.  On a small mesh
+// the one-lane kernels leave most SMs a warp or two, and what a warp takes is the
+// length of one thread's work; the operations and their order are the same.
+__device__ __forceinline__ double comp(const d4* p, const int k) { return ldw(reinterpret_cast<const double*>(p) + k); }
+__device__ __forceinline__ float comp(const float4* p, const int k) { return ldw(reinterpret_cast<const float*>(p) + k); }
+template <class T> __device__ __forceinline__ T pick_k(const T* v, const int k) {
+    return k == 0 ? v[0] : (k == 1 ? v[1] : (k == 2 ? v[2] : v[3]));
+}
+template <class T, class S, bool SECOND>
+__global__ void __launch_bounds__(128) k_prep4(const KM<T> m, const V4<S>* q, T* __restrict__ gx, T* __restrict__ gy,
+                                               T* __restrict__ phi, const Ctrl* ctrl) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, i = t >> 2, k = t & 3;
+    const bool in = i < m.n_cells;
+    int4 sl = make_int4(0, 0, 0, 0), nb = sl;
+    T A = T(1);
+    if (in) {
+        sl = __ldg(&m.cslot[i]);
+        nb = __ldg(&m.cnbr[i]);
+        A = __ldg(&m.area[i]);
+    }
+    pdl_wait();
+    if (!in || ldw(&ctrl->done)) return;
+    const T qi = comp(&q[i], k);
+    T sgx = T(0), sgy = T(0), qmn = qi, qmx = qi, dxs[4], dys[4];
+    T far[4];  // least squares: the ghost function's value of each slot
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        const int fs = pick(sl, s);
+        dxs[s] = dys[s] = far[s] = T(0);
+        if (fs == 0) continue;
+        const bool own0 = fs > 0;
+        const int f = (own0 ? fs : -fs) - 1;
+        const int o = pick(nb, s);
+        const V2<T> n = __ldg(&m.fn[f]);
+        T qo, qRv, half = T(1);
+        bool use = true;
+        if (o >= 0) {
+            qo = comp(&q[o], k);
+            qRv = qi + qo;
+            half = T(0.5);
+        } else {
+            const int bt = __ldg(&m.btype[-o - 1]);
+            T qf[4], qb[4], qR[4];
+            ldw4(&q[i], qf);
+            ld4c<T>(&m.bq[-o - 1], qb);
+            ghost_state(bt, m.gamma, n.x, n.y, qf, qb, qR);
+            qo = pick_k(qb, k);
+            qRv = pick_k(qR, k);
+            use = bt != BT_SLIP && bt != BT_WALL;
+        }
+        if (m.lsq) {
+            far[s] = o >= 0 ? qRv * T(0.5) : qRv;
+        } else {
+            const V2<T> Lg = __ldg(&m.fLg[f]);
+            const T g = Lg.y;
+            const T fk = ((own0 ? qi : qo) * (T(1) - g) + qRv * (half * g)) * Lg.x;
+            sgx += fk * flip(n.x, !own0);
+            sgy += fk * flip(n.y, !own0);
+        }
+        if (SECOND) {
+            if (use) {
+                qmn = smin(qmn, qo);
+                qmx = smax(qmx, qo);
+            }
+            const V2<T> d = own0 ? __ldg(&m.fd0[f]) : __ldg(&m.fd1[f]);
+            dxs[s] = d.x;
+            dys[s] = d.y;
+        }
+    }
+    T gxi, gyi;
+    if (m.lsq) {
+        const int code = __ldg(&m.lsqs[i]);
+        const int nj = code >> 8;
+        gxi = gyi = T(0);
+#pragma unroll 1
+        for (int j = 0; j < nj; ++j) {
+            const V2<T> w = __ldg(&m.lsqw[4 * i + j]);
+            const T d = qi - pick_k(far, (code >> (2 * j)) & 3);
+            gxi += w.x * d;
+            gyi += w.y * d;
+        }
+    } else {
+        const Div<T> iA(A);
+        gxi = iA(sgx);
+        gyi = iA(sgy);
+    }
+    gx[t] = gxi;
+    gy[t] = gyi;
+    if (SECOND)
+        phi[t] = limiter_of(m.limiter, slots_of(sl), qmx - qi, qmn - qi, gxi, gyi, dxs, dys, limiter_K3(m.limk, A));
+}
+
+template <class T, class S>
+__global__ void __launch_bounds__(128) k_limiter4(const KM<T> m, const V4<S>* qk, const T* __restrict__ gx,
+                                                  const T* __restrict__ gy, T* __restrict__ phi, const Ctrl* ctrl) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, i = t >> 2, k = t & 3;
+    const bool in = i < m.n_cells;
+    int4 sl = make_int4(0, 0, 0, 0), nb = sl;
+    T gxi = T(0), gyi = T(0), K3a = T(0), dxs[4], dys[4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) dxs[s] = dys[s] = T(0);
+    if (in) {
+        sl = __ldg(&m.cslot[i]);
+        nb = __ldg(&m.cnbr[i]);
+        gxi = __ldg(&gx[t]);
+        gyi = __ldg(&gy[t]);
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const int fs = pick(sl, s);
+            if (fs == 0) continue;
+            const V2<T> d = fs > 0 ? __ldg(&m.fd0[fs - 1]) : __ldg(&m.fd1[-fs - 1]);
+            dxs[s] = d.x;
+            dys[s] = d.y;
+        }
+        K3a = limiter_K3(m.limk, __ldg(&m.area[i]));
+    }
+    pdl_wait();
+    if (!in || ldw(&ctrl->done)) return;
+    const T qi = comp(&qk[i], k);
+    T qmn = qi, qmx = qi;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        if (pick(sl, s) == 0) continue;
+        const int o = pick(nb, s);
+        T qo;
+        if (o >= 0) {
+            qo = comp(&qk[o], k);
+        } else {
+            const int bt = __ldg(&m.btype[-o - 1]);
+            if (bt == BT_SLIP || bt == BT_WALL) continue;
+            T qb[4];
+            ld4c<T>(&m.bq[-o - 1], qb);
+            qo = pick_k(qb, k);
+        }
+        qmn = smin(qmn, qo);
+        qmx = smax(qmx, qo);
+    }
+    phi[t] = limiter_of(m.limiter, slots_of(sl), qmx - qi, qmn - qi, gxi, gyi, dxs, dys, K3a);
 }
 
 // Second-order reconstruction of one side, solver.h:780-781:
