@@ -47,3 +47,21 @@ def test_implicit_solution_on_both_sides_of_the_line(afx, ns, nr):
         assert err <= 1e-10, (prec, it, err)
         out.append(g.get_q())
     assert rel_l2(out[1], out[0]) < 1e-8
+
+
+@pytest.mark.parametrize("ns, nr", [(33, 17), (301, 151)])
+@pytest.mark.parametrize("gradient", ["green-gauss", "least-squares"])
+def test_deformed_mesh_reaches_the_fp32_slot_records(afx, ns, nr, gradient):
+    """Moving the wall by 1e-2 renews the geometry that FP32-mixed keeps per cell
+    slot: one iteration agrees with FP64's as on the mesh it was created on."""
+    m, bcs = omesh_case(ns, nr, mach=0.4, split=False)
+    out = []
+    for prec in ("fp64", "fp32-mixed"):
+        g = gpu_solver(afx, m, bcs, prec, gradient=gradient)
+        g.init()
+        q = np.array(g.get_q())
+        g.set_q(q * (1.0 + 0.01 * np.random.default_rng(4).standard_normal(q.size)))
+        g.deform_patch(np.full(len(g.patch_nodes("wall")[0]), 1e-2), "wall")
+        g.iterate(1)
+        out.append(g.get_q())
+    assert rel_l2(out[1], out[0]) < 2e-6
