@@ -146,8 +146,8 @@ def algorithmic_bytes(kernel, n, f, precision):
         # q, cslot + cnbr, area; n, (L, g), d0, d1; writes gx, gy, phi (+dt for the gather variant)
         return n * (cv + 32 + w + 3 * cv) + f * 8 * w
     if kernel == "k_limiter":
-        # qk, gx, gy, cslot + cnbr, area; d0, d1; writes phi
-        return n * (4 * cv + 32 + w) + f * 4 * w
+        # qk, gx, gy, cnbr (FP64: + cslot), area; d0, d1 (FP32: the two cells' own copies); writes phi
+        return n * (4 * cv + (32 if precision == "fp64" else 16) + w) + f * 4 * w
     return 0
 
 
