@@ -360,7 +360,9 @@ def run_gpu(args):
                                      peak_tflops=fp64_peak, frac=ops / (sec / K) / 1e12 / fp64_peak if fp64_peak else None,
                                      peak_source="measured live: FP64 FMA chains (afx_measure_fp64_peak), "
                                                  "2 flops per FMA; the bit-exact path is compiled without FMA "
-                                                 "contraction, so at most half of it is reachable")
+                                                 "contraction, so at most half of it is reachable on the FP64 "
+                                                 "pipe; quotients, roots and a share of the products are formed "
+                                                 "on the integer lanes beside it")
         result[precision] = entry
         del g
     return dict(N=N, F=F, setup_s=setup_s, res=result, fp64_peak=fp64_peak)
