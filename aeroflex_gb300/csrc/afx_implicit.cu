@@ -1285,8 +1285,10 @@ ImplicitEngine* implicit_create(const StepArgs& a, bool f32, bool graph, const s
     // over the rows with a neighbour of a higher colour, as long as one block
     // does them faster than the launches they save.  In FP64 one SM's two lanes
     // need 1.5 us for 64 rows (with 600 rows in the tail a step at 16k rows
-    // took 12 us longer)
-    const int TAIL_ROWS = e->f32 ? 640 : 64;
+    // took 12 us longer); in FP32 a tail of 640 rows in dependent stages is
+    // slower than its launches too (six iterations at 16k rows 106.6 ms, 97.7
+    // with 64 and with 200; 201k rows, Spalart-Allmaras, 12.5 against 12.2 ms)
+    const int TAIL_ROWS = 64;
     std::vector<int> blist;
     auto higher = [&](int c) {
         std::vector<int> rows;
