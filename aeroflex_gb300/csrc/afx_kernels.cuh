@@ -1306,7 +1306,13 @@ __global__ void __launch_bounds__(256) k_uniform(const KM<T> m, const V4<S>* __r
 // for 18 us; one block per case took 22): every block its share, four
 // accumulators per thread (several loads in flight), a fixed-order block sum,
 // then the blocks' sums in order.  Thread 0 of every block gets the total.
+// A block's shared memory may be written by another only once that block has
+// started, which a cluster barrier alone says: the kernel arrives at it first
+// of all (cluster_arrive), and the wait for it stands before the first remote
+// store, behind the block's own sum.  A block that leaves early waits too.
 constexpr int CASE_CTAS = 8, CASE_THREADS = 256;
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait;" ::: "memory"); }
 __device__ __forceinline__ double case_sum(const double* cell_sq, const int b0, const int b1, double* sh,
                                            double* parts) {
     namespace cg = cooperative_groups;
@@ -1323,6 +1329,7 @@ __device__ __forceinline__ double case_sum(const double* cell_sq, const int b0, 
     }
     for (; k < e; k += st) v0 += ldw(&cell_sq[k]);
     const double t = block_sum((v0 + v1) + (v2 + v3), sh);
+    cluster_wait();  // every block of the cluster has started
     if (threadIdx.x < CASE_CTAS) {
         // thread 0's sum into slot `rank` of every block of the cluster
         const double mine = __shfl_sync((1u << CASE_CTAS) - 1u, t, 0);
@@ -1342,10 +1349,14 @@ static __global__ void __cluster_dims__(CASE_CTAS, 1, 1) __launch_bounds__(CASE_
     k_case_control(const double* cell_sq, const int* __restrict__ case_off, CaseCtrl* cctrl, int* case_done,
                    double* chist, Ctrl* ctrl, int n_cases, int uniform) {
     __shared__ double sh[32], parts[CASE_CTAS];
+    cluster_arrive();
     pdl_wait();
     const int c = blockIdx.x / CASE_CTAS;
     CaseCtrl& cc = cctrl[c];
-    if (!uniform && (ldw(&ctrl->done) || ldw(&cc.done))) return;  // the whole cluster alike
+    if (!uniform && (ldw(&ctrl->done) || ldw(&cc.done))) {  // the whole cluster alike
+        cluster_wait();
+        return;
+    }
     const double t = case_sum(cell_sq, __ldg(&case_off[c]), __ldg(&case_off[c + 1]), sh, parts);
     if (blockIdx.x % CASE_CTAS != 0 || threadIdx.x != 0) return;
     const double norm = sqrt(t);
@@ -1385,12 +1396,15 @@ static __global__ void __cluster_dims__(CASE_CTAS, 1, 1) __launch_bounds__(CASE_
                      Ctrl* ctrl, d4* __restrict__ b) {
     __shared__ double sh[32], parts[CASE_CTAS];
     __shared__ int bad;
+    cluster_arrive();
     pdl_wait();
     const int c = blockIdx.x / CASE_CTAS, rank = blockIdx.x % CASE_CTAS;
-    if (ldw(&cctrl[c].done)) return;  // the whole cluster alike
+    if (ldw(&cctrl[c].done)) {  // the whole cluster alike
+        cluster_wait();
+        return;
+    }
     const int b0 = __ldg(&case_off[c]), b1 = __ldg(&case_off[c + 1]);
-    const double t = case_sum(cell_sq, b0, b1, sh, parts);
-    cooperative_groups::this_cluster().sync();  // every block has read cctrl[c].done
+    const double t = case_sum(cell_sq, b0, b1, sh, parts);  // its barrier: every block has read cctrl[c].done
     if (threadIdx.x == 0) {
         bad = !(t == t) || t > 1.7976931348623157e308;
         if (bad && rank == 0) {
