@@ -665,35 +665,32 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
     return t;
 }
 
-// The same over a block's FP32 values, as unevaluated pairs on the FP32 lanes
-// (the sum is good to 48 bits; shuffled doubles took five FP64 additions per
-// warp).  sh: 64 floats' worth.
-__device__ __forceinline__ double block_sum_f32(const float v, double* sh) {
-    float h = v, l = 0.f;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-        pair_add(h, l, __shfl_down_sync(0xffffffffu, h, o), __shfl_down_sync(0xffffffffu, l, o));
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    float2* s = reinterpret_cast<float2*>(sh);
-    if (lane == 0) s[w] = make_float2(h, l);
+// The same over a block's FP32 values: every sum in double, as block_sum's, by
+// one warp -- for 256 values 12 FP64 additions of a warp, where shuffling
+// doubles in all eight warps takes 40 and more.
+__device__ __forceinline__ double block_sum_f32(const float v) {
+    __shared__ float s[256];
+    s[threadIdx.x] = v;
     __syncthreads();
-    if (threadIdx.x != 0) return 0.0;
-    h = l = 0.f;
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) pair_add(h, l, s[k].x, s[k].y);
-    return (double)h + (double)l;
+    if (threadIdx.x >= 32) return 0.0;
+    double t = fp64::widen(__float_as_uint(s[threadIdx.x]));
+    for (int k = threadIdx.x + 32; k < (int)blockDim.x; k += 32) t += fp64::widen(__float_as_uint(s[k]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    return t;
 }
 
 // FP32-mixed epilogue.  GB300's FP64 pipe issues at ~1/64 of the FP32 rate,
 // so FP64 is spent only where it accumulates, in the four additions to the state
-// (conversions are integer arithmetic, the norm's sum pairs of FP32: with both
-// on the FP64 pipe some 20 of its instructions per warp made the last stage
-// 220 us at 4.19M cells, 170 now): the RK increment
+// and in the norm's sums (conversions are integer arithmetic and one warp adds a
+// block's squares: with both on the FP64 pipe in every warp some 20 of its
+// instructions per warp made the last stage 220 us at 4.19M cells): the RK increment
 // R*dt*alpha*relaxation is formed in FP32; the intermediate stage states
 // (which only feed FP32 fluxes) are q_shadow + increment in FP32; the new
 // state of the last stage is q (FP64) + increment in FP64, and its FP32
 // shadow is re-rounded from the FP64 result every iteration, so FP32
 // rounding never accumulates in the state.  The norm sums per-cell FP32
-// squares as unevaluated pairs in a block and in FP64 over the blocks.
+// squares in FP64.
 template <class S>
 __device__ __forceinline__ void stage_epilogue_mixed(const StageOut<float, S>& o, const int i, const float* R0,
                                                      const float dti, float& sq) {
@@ -825,7 +822,7 @@ __device__ __forceinline__ void stage_epilogue(const StageOut<T, S>& o, const in
         }
     }
     if (sizeof(T) == 4 && o.mode == 1 && !__syncthreads_or(fp64::bits_of(sq) != 0)) {
-        const double t = block_sum_f32(sqf, sh);
+        const double t = block_sum_f32(sqf);
         if (threadIdx.x == 0) o.partials[blockIdx.x] = t;
     } else if (o.mode == 1 || o.mode == 3) {
         if (sizeof(T) == 4) sq += (double)sqf;  // with the squares of frozen ghosts
