@@ -89,12 +89,11 @@ __device__ __forceinline__ float to_f32(const double x) {
 __device__ __forceinline__ void st4(float4* p, const double* v) {
     *p = make_float4(to_f32(v[0]), to_f32(v[1]), to_f32(v[2]), to_f32(v[3]));
 }
-// (h, l) += (oh, ol), unevaluated pairs: Knuth's two-sum of the leading parts
-__device__ __forceinline__ void pair_add(float& h, float& l, const float oh, const float ol) {
-    const float s = __fadd_rn(h, oh), b = __fadd_rn(s, -h);
-    const float err = __fadd_rn(__fadd_rn(h, -__fadd_rn(s, -b)), __fadd_rn(oh, -b));
-    l = __fadd_rn(__fadd_rn(l, ol), err);
-    h = s;
+// a + b and the error of it, exactly (Knuth's two-sum)
+__device__ __forceinline__ float two_sum(const float a, const float b, float& err) {
+    const float s = __fadd_rn(a, b), c = __fadd_rn(s, -a);
+    err = __fadd_rn(__fadd_rn(a, -__fadd_rn(s, -c)), __fadd_rn(b, -c));
+    return s;
 }
 
 __device__ __forceinline__ double dsqrt(double x) { return fp64::root(x); }

@@ -697,8 +697,8 @@ __global__ void __launch_bounds__(128) k_imp_next_vec(const Ell e, const int n_r
 // butterfly that halves the outputs a lane holds at every step takes 31 (16
 // for up to 16 outputs) additions of a warp instead of 5 per output -- in
 // FP64 each of them holds the FP64 pipe for 18.6 cycles, and this reduction
-// was most of the kernel.  FP32 sums are added as unevaluated pairs (error-free
-// two-sum, 48 bits) on the FP32 lanes; double takes over after it.  Each block
+// was most of the kernel.  FP32 sums are added as unevaluated triples (error-free
+// two-sums, 72 bits) on the FP32 lanes; double takes over after it.  Each block
 // writes its partial sums; the last block to finish adds them in a fixed
 // pattern (a warp per group of blocks, then over the warps), so the result is
 // deterministic, and re-arms the counter.
@@ -717,50 +717,82 @@ __device__ __forceinline__ void vsub(double2& w, const double h, const double2 v
     w.x -= h * v.x; w.y -= h * v.y;
 }
 
-// A partial sum on its way through the warp's reduction
-template <class T> struct Part;
-template <> struct Part<double> {
-    double v;
-    __device__ __forceinline__ void set(const double a) { v = a; }
-    __device__ __forceinline__ double get() const { return v; }
-    __device__ __forceinline__ Part from(const int m) const {
-        Part o;
-        o.v = __shfl_xor_sync(0xffffffffu, v, m);
-        return o;
-    }
-    __device__ __forceinline__ void add(const Part& o) { v += o.v; }
-};
-template <> struct Part<float> {
-    float h, l;  // unevaluated sum
-    __device__ __forceinline__ void set(const float a) { h = a; l = 0.f; }
-    __device__ __forceinline__ double get() const { return (double)h + (double)l; }
-    __device__ __forceinline__ Part from(const int m) const {
-        Part o;
-        o.h = __shfl_xor_sync(0xffffffffu, h, m);
-        o.l = __shfl_xor_sync(0xffffffffu, l, m);
-        return o;
-    }
-    __device__ __forceinline__ void add(const Part& o) { pair_add(h, l, o.h, o.l); }
-};
 // Sums of acc[0..W-1] over the warp; lane j (mod W) gets output j
-template <int W, class T>
-__device__ __forceinline__ Part<T> warp_sums(const T* acc, const int lane) {
-    Part<T> a[W];
+template <int W>
+__device__ __forceinline__ double warp_sums(const double* acc, const int lane) {
+    double a[W];
 #pragma unroll
-    for (int j = 0; j < W; ++j) a[j].set(acc[j]);
+    for (int j = 0; j < W; ++j) a[j] = acc[j];
 #pragma unroll
     for (int m = W / 2; m > 0; m >>= 1) {
         const bool up = lane & m;
 #pragma unroll
         for (int j = 0; j < m; ++j) {
-            const Part<T> give = up ? a[j] : a[j + m];
-            a[j] = up ? a[j + m] : a[j];
-            a[j].add(give.from(m));
+            const double give = up ? a[j] : a[j + m];
+            a[j] = (up ? a[j + m] : a[j]) + __shfl_xor_sync(0xffffffffu, give, m);
         }
     }
 #pragma unroll
-    for (int m = W; m < 32; m <<= 1) a[0].add(a[0].from(m));
+    for (int m = W; m < 32; m <<= 1) a[0] += __shfl_xor_sync(0xffffffffu, a[0], m);
     return a[0];
+}
+// Unevaluated sum h + m + l of FP32 numbers, level by level of the butterfly:
+// two numbers give an exact pair, two pairs an exact triple but for 2^-72, and so
+// on, so the sum of the warp has all the bits a double holds.
+struct Triple {
+    float h, m, l;
+    __device__ __forceinline__ Triple from(const int lane_mask, const int level) const {
+        Triple o;
+        o.h = __shfl_xor_sync(0xffffffffu, h, lane_mask);
+        o.m = level > 0 ? __shfl_xor_sync(0xffffffffu, m, lane_mask) : 0.f;
+        o.l = level > 1 ? __shfl_xor_sync(0xffffffffu, l, lane_mask) : 0.f;
+        return o;
+    }
+    __device__ __forceinline__ void add(const Triple& o, const int level) {
+        float e, e1, e2;
+        h = two_sum(h, o.h, e);
+        if (level == 0) {
+            m = e;
+            return;
+        }
+        m = two_sum(m, o.m, e1);
+        m = two_sum(m, e, e2);
+        l = level > 1 ? (l + o.l) + (e1 + e2) : e1 + e2;
+    }
+};
+template <int W>
+__device__ __forceinline__ double warp_sums(const float* acc, const int lane) {
+    // a double would hold any sum of these, so they are brought to the middle of
+    // FP32's range if one could overflow, or if all are so small that the last
+    // parts could underflow
+    float mx = 0.f;
+#pragma unroll
+    for (int j = 0; j < W; ++j) mx = fmaxf(mx, fabsf(acc[j]));
+    mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx)));
+    const float sc = mx > 0x1p122f ? 0x1p-6f : (mx < 0x1p-40f && mx > 0.f ? 0x1p100f : 1.f);
+    Triple a[W];
+#pragma unroll
+    for (int j = 0; j < W; ++j) a[j] = Triple{acc[j], 0.f, 0.f};
+    if (sc != 1.f) {
+#pragma unroll
+        for (int j = 0; j < W; ++j) a[j].h *= sc;
+    }
+    int level = 0;
+#pragma unroll
+    for (int m = W / 2; m > 0; m >>= 1, ++level) {
+        const bool up = lane & m;
+#pragma unroll
+        for (int j = 0; j < m; ++j) {
+            const Triple give = up ? a[j] : a[j + m];
+            a[j] = up ? a[j + m] : a[j];
+            a[j].add(give.from(m, level), level);
+        }
+    }
+#pragma unroll
+    for (int m = W; m < 32; m <<= 1, ++level) a[0].add(a[0].from(m, level), level);
+    // (an infinity or a NaN among the summands: h alone is their sum)
+    const double t = fabsf(a[0].h) <= 3.402823466e38f ? ((double)a[0].l + (double)a[0].m) + (double)a[0].h : (double)a[0].h;
+    return sc == 1.f ? t : t * (sc < 1.f ? 0x1p6 : 0x1p-100);
 }
 
 // Arnoldi step j = c->k, classical Gram-Schmidt twice: h1 (first pass) and
@@ -837,14 +869,14 @@ __device__ __forceinline__ bool grid_sums(const T* acc, const int nout, const in
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     if (adds) {
         if (ONE) {
-            const Part<T> v = warp_sums<1, T>(acc, lane);
-            if (lane == 0) sh[wp][0] = v.get();
+            const double v = warp_sums<1>(acc, lane);
+            if (lane == 0) sh[wp][0] = v;
         } else if (nout > 16) {
-            const Part<T> v = warp_sums<32, T>(acc, lane);
-            if (lane < nout) sh[wp][lane] = v.get();
+            const double v = warp_sums<32>(acc, lane);
+            if (lane < nout) sh[wp][lane] = v;
         } else {
-            const Part<T> v = warp_sums<16, T>(acc, lane);
-            if (lane < nout) sh[wp][lane] = v.get();
+            const double v = warp_sums<16>(acc, lane);
+            if (lane < nout) sh[wp][lane] = v;
         }
     }
     __syncthreads();
