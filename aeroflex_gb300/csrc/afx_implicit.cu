@@ -689,10 +689,11 @@ __global__ void __launch_bounds__(128) k_imp_next_vec(const Ell e, const int n_r
 //   k_imp_next_vec    w -= V h2, scaled to v_{k+1}, by the next step
 // The norm after the second update comes from Pythagoras, w.w - h2.h2 (the
 // basis is orthonormal and h2 a rounding correction), so the second update
-// needs no reduction of its own.  (Were it inaccurate, as it is at a
-// breakdown, v_{k+1} would not have unit length, but the Arnoldi relation
-// would still hold: the vector is divided by the same number that enters the
-// matrix.)
+// needs no reduction of its own.  Where h2.h2 is more than half of w.w -- near
+// a breakdown, the first update left mostly rounding -- the difference would
+// lose digits, down to a zero that ends the solve as converged: there the last
+// block forms the updated vector and its norm.  Up to a half the difference is
+// good to five units of the vectors' rounding.
 // The per-thread sums of all outputs are reduced across a warp together: a
 // butterfly that halves the outputs a lane holds at every step takes 31 (16
 // for up to 16 outputs) additions of a warp instead of 5 per output -- in
@@ -812,15 +813,11 @@ __device__ __forceinline__ void givens_stage(const GmresCtl* c, const double* h1
         g.sn[t] = ldw(&c->sn[t]);
     }
 }
-__device__ __forceinline__ void givens(GmresCtl* c, const double h2, const double sq, GivensCol& g, double* scale) {
+__device__ __forceinline__ void givens(GmresCtl* c, const double h2, const double ww, GivensCol& g, double* scale) {
     using namespace fp64;
     const int lane = threadIdx.x, j = c->k;
-    // sq: w.w after the first update in lane j + 1; h2 in lanes 0..j
+    // ww: the squared norm after the second update; h2 in lanes 0..j
     if (lane <= j) g.col[lane] += h2;
-    double hh = lane <= j ? h2 * h2 : 0.0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) hh += __shfl_xor_sync(0xffffffffu, hh, o);
-    const double ww = __shfl_sync(0xffffffffu, sq, j + 1) - hh;
     __syncwarp();
     if (lane == 0) {
         const double gj = c->g[j], tol = c->tol;
@@ -922,6 +919,30 @@ __device__ __forceinline__ bool grid_sums(const T* acc, const int nout, const in
     return true;
 }
 
+// Squared norm of w - sum_j h2_j v_j by one block (thread j holds h2_j, hs is
+// overwritten with them); for the threads of the first warp.  w as the whole
+// grid has left it.  Rare: out of line.
+template <class T>
+__device__ __noinline__ double updated_norm(const int nc, const int nv, const typename Vec16<T>::type* V,
+                                            const typename Vec16<T>::type* w, const double h2, T* hs) {
+    __shared__ double sh[DOT_THREADS / 32];
+    if ((int)threadIdx.x < nv) hs[threadIdx.x] = (T)h2;
+    __syncthreads();
+    T acc[1] = {0};
+    for (int i = threadIdx.x; i < nc; i += blockDim.x) {
+        typename Vec16<T>::type wi = __ldcg(&w[i]);
+        for (int j = 0; j < nv; ++j) vsub(wi, hs[j], __ldcg(&V[(size_t)j * nc + i]));
+        acc[0] += vdot(wi, wi);
+    }
+    const double v = warp_sums<1>(acc, threadIdx.x & 31);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double t = 0;
+#pragma unroll
+    for (int k = 0; k < DOT_THREADS / 32; ++k) t += sh[k];
+    return t;
+}
+
 // w -= sum_j h1_j v_j, then h2_j = v_j . w and w.w, and in the last block the
 // step's column.  A chunk of every vector stays in registers for the second
 // product (one block per SM); the first chunk's are read ahead of the wait (the
@@ -982,9 +1003,21 @@ __global__ void __launch_bounds__(DOT_THREADS, 1) k_imp_cgs(const int n, const T
         if (j == nv) acc[j] = sq;
     double t = 0;
     const bool mine = grid_sums<T, DOT_THREADS, false>(acc, nv + 1, (int)blockIdx.x, (int)gridDim.x, part, counter, t);
-    if (!__syncthreads_or(mine) || threadIdx.x >= 32) return;
-    if ((int)threadIdx.x < nv) h2[threadIdx.x] = t;
-    givens(c, t, t, gc, scale);
+    if (!__syncthreads_or(mine)) return;
+    __shared__ bool direct;
+    double hh = 0, ww = 0;
+    if (threadIdx.x < 32) {
+        hh = (int)threadIdx.x < nv ? t * t : 0.0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) hh += __shfl_xor_sync(0xffffffffu, hh, o);
+        ww = __shfl_sync(0xffffffffu, t, nv);
+        if ((int)threadIdx.x < nv) h2[threadIdx.x] = t;
+        if (threadIdx.x == 0) direct = !(2.0 * hh <= ww);
+    }
+    __syncthreads();
+    if (direct) ww = updated_norm<T>(nc, nv, Vv, wv, t, hs);
+    else ww -= hh;
+    if (threadIdx.x < 32) givens(c, t, ww, gc, scale);
 }
 
 // out = w.w

@@ -35,11 +35,44 @@ int sq(int n, int blocks, const T* w, double* out) {
     return 0;
 }
 
+// Gram-Schmidt of w against the k + 1 vectors in V (given h1), and the step's
+// column after rotations by zero angles: h2 and {hnext, res, stop, k} come back
+template <class T>
+int cgs(int n, int k, int blocks, const T* V, T* w, const double* h1, double g, double tol, double* h2, double* st) {
+    GmresCtl c{};
+    c.k = k;
+    c.max_iters = 500;
+    c.tol = tol;
+    c.g[k] = g;
+    for (int i = 0; i < GM_M; ++i) c.cs[i] = 1.0;
+    {
+        Buf dV(V, (size_t)(k + 1) * n * sizeof(T)), dw(w, n * sizeof(T), true), dh1(h1, (k + 1) * 8);
+        Buf part(nullptr, blocks * (GM_M + 1) * 8), cnt(nullptr, 4), dh2(h2, (k + 1) * 8, true), sc(nullptr, 8);
+        Buf dc(&c, sizeof(c), true);
+        launch_pdl(k_imp_cgs<T>, blocks, DOT_THREADS, 0, nullptr, n, dV.p<T>(), dw.p<T>(), dh1.p<double>(),
+                   part.p<double>(), cnt.p<unsigned>(), dh2.p<double>(), dc.p<GmresCtl>(), sc.p<double>());
+        if (cudaDeviceSynchronize() != cudaSuccess) return 1;
+    }
+    st[0] = c.hnext;
+    st[1] = c.res;
+    st[2] = c.stop;
+    st[3] = c.k;
+    return 0;
+}
+
 }  // namespace
 
 extern "C" {
 
 int hk_sq_f32(int n, int blocks, const float* w, double* out) { return sq<float>(n, blocks, w, out); }
 int hk_sq_f64(int n, int blocks, const double* w, double* out) { return sq<double>(n, blocks, w, out); }
+int hk_cgs_f32(int n, int k, int blocks, const float* V, float* w, const double* h1, double g, double tol, double* h2,
+               double* st) {
+    return cgs<float>(n, k, blocks, V, w, h1, g, tol, h2, st);
+}
+int hk_cgs_f64(int n, int k, int blocks, const double* V, double* w, const double* h1, double g, double tol,
+               double* h2, double* st) {
+    return cgs<double>(n, k, blocks, V, w, h1, g, tol, h2, st);
+}
 
 }  // extern "C"

@@ -54,3 +54,36 @@ def test_norms_against_64_bits(hk, n, blocks):
     assert abs(_sq(hk, w, blocks) - w @ w) <= 1e-14 * (w @ w)
     f = np.trunc(np.clip(w, -4.0, 4.0) * 2 ** 7).astype(np.float32)
     assert _sq(hk, f, blocks) == float((f.astype(np.float64) ** 2).sum())
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("k", [0, 3, 15, 16, 29])
+@pytest.mark.parametrize("cells, blocks", [(60, 1), (3000, 12), (3000, 5)])
+@pytest.mark.parametrize("near", [False, True])
+def test_norm_of_the_new_vector_near_a_breakdown(hk, dtype, k, cells, blocks, near):
+    """A product that lies in the span of the basis but for delta p (near): the
+    first Gram-Schmidt pass leaves 1e-3 of it and the second has to find delta.
+    The vector after the second pass is formed with a rounding per term, so its
+    norm is good to (k + 3) units of the first remainder's; and since the last
+    component is zero, the step gains nothing and the solve must not end."""
+    rng = np.random.default_rng(cells + k)
+    n, u = 4 * cells, float(np.finfo(dtype).eps)
+    Q = np.linalg.qr(rng.standard_normal((n, k + 2)))[0]
+    V = np.ascontiguousarray(Q[:, : k + 1].T.astype(dtype))
+    c = rng.standard_normal(k + 1)
+    c[k] = 0.0
+    delta = u if near else 0.3
+    w = (Q[:, : k + 1] @ c + delta * Q[:, k + 1]).astype(dtype)
+    h1 = c * 1.001 if near else V.astype(np.float64) @ w.astype(np.float64)
+    w0 = w.astype(np.float64)
+    h2, st = np.zeros(k + 1), np.zeros(4)
+    fn = hk.hk_cgs_f32 if dtype == np.float32 else hk.hk_cgs_f64
+    w1 = w.copy()
+    assert fn(n, k, blocks, _p(V), _p(w1), _p(h1), ctypes.c_double(1.0), ctypes.c_double(1e-2), _p(h2), _p(st)) == 0
+    first = w1.astype(np.float64)  # after the first pass, as the kernel left it
+    assert np.abs(first - (w0 - h1 @ V.astype(np.float64))).max() <= 2 * (k + 3) * u * np.abs(h1).max(initial=1.0)
+    ref = np.linalg.norm(first - h2 @ V.astype(np.float64))
+    assert abs(st[0] - ref) <= (k + 3) * u * np.linalg.norm(first)
+    assert st[3] == k + 1
+    if near and ref > 0.0:
+        assert st[1] > 0.5 and st[2] == (1.0 if k == 29 else 0.0)
