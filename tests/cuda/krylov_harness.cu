@@ -60,9 +60,36 @@ int cgs(int n, int k, int blocks, const T* V, T* w, const double* h1, double g, 
     return 0;
 }
 
+// One colour (rows c0 .. c0 + n - 1) of the sweep over x, with rt threads per row
+template <class T>
+int gs(int rt, int N, int c0, int n, int fwd, const int* col, const T* dinv, const T* off, const T* r, T* x) {
+    {
+        Buf dc(col, N * sizeof(int4)), di(dinv, 16 * (size_t)N * sizeof(T)), dof(off, 64 * (size_t)N * sizeof(T));
+        Buf dr(r, 4 * (size_t)N * sizeof(T)), dx(x, 4 * (size_t)N * sizeof(T), true);
+        const Ell e{nullptr, dc.p<int4>(), nullptr, nullptr, nullptr};
+        if (rt == 4)
+            launch_pdl(k_imp_gs<T, 4>, nb_(4LL * n, 128), 128, 0, nullptr, e, N, di.p<T>(), dof.p<T>(), c0, n, dr.p<T>(),
+                       nullptr, 0LL, dx.p<T>(), nullptr, nullptr, fwd != 0);
+        else
+            launch_pdl(k_imp_gs<T, 1>, nb_(n, 128), 128, 0, nullptr, e, N, di.p<T>(), dof.p<T>(), c0, n, dr.p<T>(),
+                       nullptr, 0LL, dx.p<T>(), nullptr, nullptr, fwd != 0);
+        if (cudaDeviceSynchronize() != cudaSuccess) return 1;
+    }
+    return 0;
+}
+
 }  // namespace
 
 extern "C" {
+
+int hk_gs_f32(int rt, int N, int c0, int n, int fwd, const int* col, const float* dinv, const float* off, const float* r,
+              float* x) {
+    return gs<float>(rt, N, c0, n, fwd, col, dinv, off, r, x);
+}
+int hk_gs_f64(int rt, int N, int c0, int n, int fwd, const int* col, const double* dinv, const double* off,
+              const double* r, double* x) {
+    return gs<double>(rt, N, c0, n, fwd, col, dinv, off, r, x);
+}
 
 int hk_sq_f32(int n, int blocks, const float* w, double* out) { return sq<float>(n, blocks, w, out); }
 int hk_sq_f64(int n, int blocks, const double* w, double* out) { return sq<double>(n, blocks, w, out); }

@@ -87,3 +87,33 @@ def test_norm_of_the_new_vector_near_a_breakdown(hk, dtype, k, cells, blocks, ne
     assert st[3] == k + 1
     if near and ref > 0.0:
         assert st[1] > 0.5 and st[2] == (1.0 if k == 29 else 0.0)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("threads", [1, 4])
+@pytest.mark.parametrize("fwd", [0, 1])
+@pytest.mark.parametrize("n", [1, 31, 129, 45000])
+def test_one_colour_of_the_sweep(hk, dtype, threads, fwd, n):
+    """x_p = D_p^-1 (r_p - sum O x_q) over one colour's rows, with one thread per
+    row (colours of 40,000 rows and more) and with four, against 64 bits: up to
+    sixteen products and a 4 x 4 block, forty roundings of terms of at most 4 + 16."""
+    rng = np.random.default_rng(n + fwd)
+    lo = max(n // 3, 8)  # rows of lower and of higher colours beside the colour's own
+    N, c0 = n + 2 * lo, lo
+    other = np.concatenate([np.arange(c0), np.arange(c0 + n, N)])
+    col = np.where(rng.random((N, 4)) < 0.2, -1, rng.choice(other, (N, 4))).astype(np.int32)
+    dinv, off = rng.uniform(-1, 1, (N, 4, 4)).astype(dtype), rng.uniform(-1, 1, (N, 4, 4, 4)).astype(dtype)
+    r, x0 = rng.uniform(-1, 1, (N, 4)).astype(dtype), rng.uniform(-1, 1, (N, 4)).astype(dtype)
+    # interleaved: 16-byte chunk c of slot s of row p is chunk (s * chunks + c) * N + p
+    w = 16 // np.dtype(dtype).itemsize
+    packed = np.ascontiguousarray(off.reshape(N, 4, 16 // w, w).transpose(1, 2, 0, 3))
+    x = x0.copy()
+    fn = hk.hk_gs_f32 if dtype == np.float32 else hk.hk_gs_f64
+    assert fn(threads, N, c0, n, fwd, _p(col), _p(dinv), _p(packed), _p(r), _p(x)) == 0
+    use = (col >= 0) & ((col < c0) if fwd else True)
+    xo = np.where(use[..., None], x0[col].astype(np.float64), 0.0)
+    s = r - np.einsum("pkij,pkj->pi", off.astype(np.float64), xo)
+    ref = x0.astype(np.float64)
+    ref[c0 : c0 + n] = np.einsum("pij,pj->pi", dinv.astype(np.float64), s)[c0 : c0 + n]
+    assert np.abs(x - ref).max() <= 40 * np.finfo(dtype).eps * 20 * 4
+    np.testing.assert_array_equal(np.delete(x, np.s_[c0 : c0 + n], 0), np.delete(x0, np.s_[c0 : c0 + n], 0))
