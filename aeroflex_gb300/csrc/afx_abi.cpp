@@ -1126,6 +1126,9 @@ static std::unique_ptr<afx_solver_s> make_solver(const HostMesh& m, const Device
         a.n_cells = L.n_cells;
         a.n_faces = L.n_faces;
         a.n_bnd = L.n_bnd;
+        int device = 0;
+        AFX_CUDA(cudaGetDevice(&device));
+        AFX_CUDA(cudaDeviceGetAttribute(&a.sms, cudaDevAttrMultiProcessorCount, device));
         const size_t N = L.n_cells, F = L.n_faces, B = L.n_bnd;
         a.cslot = s->dupload(L.cslot);
         a.cnbr = s->dupload(L.cnbr);

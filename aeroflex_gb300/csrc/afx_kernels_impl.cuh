@@ -13,12 +13,12 @@ KM<T> make_km(const StepArgs& a) {
     KM<T> m;
     m.n_cells = a.n_cells;
     m.n_faces = a.n_faces;
-    // the streams of a block two blocks per SM on are brought into L2 (k_prep
-    // 173 -> 154 us, k_limiter_f32 85 -> 79 us at 4.19M cells; four per SM no
-    // better, eight worse); below about a million cells the arrays stay in L2 by
-    // themselves and the requests only cost time (k_limiter, 590k cells: 15.9 ->
-    // 16.8 us)
-    m.ahead = a.n_cells >= 1000000 ? 304 : 0;
+    // the streams of the cells two blocks of 256 per SM on are brought into L2
+    // (k_prep 173 -> 154 us, k_limiter_f32 85 -> 79 us at 4.19M cells; four per SM
+    // no better, eight worse); below about a million cells the arrays stay in L2
+    // by themselves and the requests only cost time (k_limiter, 590k cells: 15.9
+    // -> 16.8 us)
+    m.ahead = a.n_cells >= 1000000 ? 2 * a.sms * 256 / a.block : 0;
     m.cslot = (const int4*)a.cslot;
     m.cnbr = (const int4*)a.cnbr;
     m.area = (const T*)a.area;

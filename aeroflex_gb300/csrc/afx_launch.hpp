@@ -130,6 +130,7 @@ struct StepArgs {
     double sa_nu_far = 0.;                 // nu~ of the far field, 3 mu_L / rho_inf
     Prof* prof = nullptr;      // eager profiling only (never inside a graph)
     bool pdl = true;           // launch as programmatic dependents (afx_pdl.cuh)
+    int sms = 0;               // multiprocessors of the device
 };
 
 // One explicit iteration reading parity p, writing parity p^1.
