@@ -853,31 +853,28 @@ __device__ __forceinline__ void givens(GmresCtl* c, const double h2, const doubl
 }
 
 // The block's and, in the last block to finish, the whole sum of the threads'
-// acc[0..nout-1] over blocks 0..nblk-1 of NT threads; true in the last block's
-// first nout threads, with the sums in `total`.  A block with blk < 0 only
-// counts itself.
+// acc[0..nout-1] over the grid's blocks of NT threads; true in the last block's
+// first nout threads, with the sums in `total`.
 template <class T, int NT, bool ONE>
-__device__ __forceinline__ bool grid_sums(const T* acc, const int nout, const int blk, const int nblk,
-                                          double* part, unsigned* counter, double& total) {
-    const bool adds = blk >= 0;
+__device__ __forceinline__ bool grid_sums(const T* acc, const int nout, double* part, unsigned* counter,
+                                          double& total) {
+    const int blk = (int)blockIdx.x, nblk = (int)gridDim.x;
     constexpr int NW = NT / 32;
     __shared__ double sh[NW][32];
     __shared__ bool last;
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-    if (adds) {
-        if (ONE) {
-            const double v = warp_sums<1>(acc, lane);
-            if (lane == 0) sh[wp][0] = v;
-        } else if (nout > 16) {
-            const double v = warp_sums<32>(acc, lane);
-            if (lane < nout) sh[wp][lane] = v;
-        } else {
-            const double v = warp_sums<16>(acc, lane);
-            if (lane < nout) sh[wp][lane] = v;
-        }
+    if (ONE) {
+        const double v = warp_sums<1>(acc, lane);
+        if (lane == 0) sh[wp][0] = v;
+    } else if (nout > 16) {
+        const double v = warp_sums<32>(acc, lane);
+        if (lane < nout) sh[wp][lane] = v;
+    } else {
+        const double v = warp_sums<16>(acc, lane);
+        if (lane < nout) sh[wp][lane] = v;
     }
     __syncthreads();
-    if (adds && (int)threadIdx.x < nout) {
+    if ((int)threadIdx.x < nout) {
         double t = 0;
 #pragma unroll
         for (int k = 0; k < NW; ++k) t += sh[k][threadIdx.x];
@@ -885,7 +882,7 @@ __device__ __forceinline__ bool grid_sums(const T* acc, const int nout, const in
         __threadfence();  // the partials are visible before the block is counted
     }
     __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
+    if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == (unsigned)nblk - 1;
     __syncthreads();
     if (!last) return false;
     __threadfence();
@@ -1002,7 +999,7 @@ __global__ void __launch_bounds__(DOT_THREADS, 1) k_imp_cgs(const int n, const T
     for (int j = 1; j < GM_M + 2; ++j)
         if (j == nv) acc[j] = sq;
     double t = 0;
-    const bool mine = grid_sums<T, DOT_THREADS, false>(acc, nv + 1, (int)blockIdx.x, (int)gridDim.x, part, counter, t);
+    const bool mine = grid_sums<T, DOT_THREADS, false>(acc, nv + 1, part, counter, t);
     if (!__syncthreads_or(mine)) return;
     __shared__ bool direct;
     double hh = 0, ww = 0;
@@ -1034,7 +1031,7 @@ __global__ void __launch_bounds__(DOT_THREADS) k_imp_sq(const int n, const T* w,
         acc[0] += vdot(wi, wi);
     }
     double t;
-    if (grid_sums<T, DOT_THREADS, true>(acc, 1, (int)blockIdx.x, (int)gridDim.x, part, counter, t)) out[0] = t;
+    if (grid_sums<T, DOT_THREADS, true>(acc, 1, part, counter, t)) out[0] = t;
 }
 
 // w = M x and out_j = v_j . w, j <= *vk, in one pass over the rows: the
@@ -1089,7 +1086,7 @@ __global__ void __launch_bounds__(DOT_THREADS, 2)
             }
     }
     double s;
-    if (grid_sums<T, DOT_THREADS, false>(acc, nv, (int)blockIdx.x, (int)gridDim.x, part, counter, s)) out[threadIdx.x] = s;
+    if (grid_sums<T, DOT_THREADS, false>(acc, nv, part, counter, s)) out[threadIdx.x] = s;
 }
 
 // Back substitution R y = g over the k steps of the cycle: one warp, a lane
