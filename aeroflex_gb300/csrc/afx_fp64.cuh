@@ -23,7 +23,7 @@
 //     product (a zero over a normal number, and a zero times a finite one, are
 //     answered here).
 // The reciprocal seeds are the hardware's single-precision approximations
-// (2 ulp allowed for) and one Newton step in 32-bit fixed point.
+// (3 ulp allowed for) and one Newton step in 32-bit fixed point.
 #pragma once
 
 #include <cstdint>

@@ -229,10 +229,12 @@ StageOut<T, S> base_out(const StepArgs& a, int p) {
 template <class T, class S, bool SHADOW>
 void iteration(const StepArgs& a0, int p, cudaStream_t s) {
     // Iterations run from a graph, which already keeps the gaps between kernels
-    // short: programmatic dependents gain 3% at 4.19M cells and cost 9% at 17k
+    // short: programmatic dependents gain on large meshes and cost on small ones
     // (blocks of the next kernel take their places while the last ones of this
-    // kernel still run).  Evaluations launched one by one (residual, rhs) gain
-    // at every size.
+    // kernel still run).  Plain over dependent time, FP32-mixed: 16k cells 0.77,
+    // 130k 0.76, 262k 0.98, 360k 1.02, 518k 1.03, 1.05M 1.03; FP64: 16k 0.86,
+    // 130k 0.96, from 262k on 1.00.  Evaluations launched one by one (residual,
+    // rhs) gain at every size.
     StepArgs a = a0;
     a.pdl = a.n_cells >= 500000;
     const KM<T> m = make_km<T>(a);
