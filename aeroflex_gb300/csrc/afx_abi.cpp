@@ -395,7 +395,7 @@ struct afx_solver_s {
             put(m->fd1, hl.fd1, f32);
             put(m->ft, hl.ft, f32);
             if (m->lsq && m->lsqw) put(m->lsqw, lw, f32);
-            if (f32) {
+            if (f32 && m->dsl) {
                 const std::vector<float> d = slot_offsets(hl);
                 AFX_CUDA(cudaMemcpyAsync((void*)m->dsl, d.data(), d.size() * 4, cudaMemcpyHostToDevice, stream));
                 AFX_CUDA(cudaStreamSynchronize(stream));
@@ -1147,7 +1147,7 @@ static std::unique_ptr<afx_solver_s> make_solver(const HostMesh& m, const Device
             a.fd0 = s->dupload(cast_vec<float>(L.fd0));
             a.fd1 = s->dupload(cast_vec<float>(L.fd1));
             a.ft = s->dupload(cast_vec<float>(L.ft));
-            a.dsl = s->dupload(slot_offsets(L));
+            if (!four_lanes(L.n_cells)) a.dsl = s->dupload(slot_offsets(L));
         }
         const size_t w = s->fp64 ? 8 : 4;
         a.btype = s->dalloc(std::max<size_t>(B, 1) * sizeof(int));

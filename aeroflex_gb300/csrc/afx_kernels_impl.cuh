@@ -58,11 +58,6 @@ inline void mark(const StepArgs& a, int id, cudaStream_t s) {
     if (a.prof) a.prof->mark(id, s);
 }
 
-// Four lanes per cell in k_prep and k_limiter?  Below 40,000 cells.  16k cells,
-// FP64: k_prep 19.7 -> 13.8 us, k_limiter 9.1 -> 6.5; 17k, FP32: 7.2 -> 4.8, 5.8 ->
-// 3.8; 74k, FP64: 44.2 against 47.7 and 16.7 against 17.3 with four.
-inline bool four_lanes(const StepArgs& a) { return a.n_cells < 40000; }
-
 template <class T, class S>
 void launch_prep(const StepArgs& a, const KM<T>& m, const V4<S>* q, cudaStream_t s) {
     const int nb = nblocks(a.n_cells, a.block);
@@ -71,7 +66,7 @@ void launch_prep(const StepArgs& a, const KM<T>& m, const V4<S>* q, cudaStream_t
     V4<T>* ph = (V4<T>*)a.phi;
     T* dt = (T*)a.dt;
     // the face and tile variants form dt in their first stage (EIG/DT)
-    if (a.variant != 0 && a.need_grad && four_lanes(a)) {
+    if (a.variant != 0 && a.need_grad && four_lanes(a.n_cells)) {
         const int n4 = nblocks(4 * a.n_cells, 128);
         if (a.second)
             launch_pdl_if(a.pdl, k_prep4<T, S, true>, n4, 128, 0, s, m, q, (T*)a.gx, (T*)a.gy, (T*)a.phi, a.ctrl);
@@ -246,7 +241,7 @@ void iteration(const StepArgs& a0, int p, cudaStream_t s) {
         const V4<S>* qk = st == 0 ? q : (const V4<S>*)a.qs[st - 1];
         if (st > 0 && a.second) {
             const int nl = nblocks(a.n_cells, a.block);
-            if (four_lanes(a))
+            if (four_lanes(a.n_cells))
                 launch_pdl_if(a.pdl, k_limiter4<T, S>, nblocks(4 * a.n_cells, 128), 128, 0, s, m, qk, (const T*)a.gx,
                               (const T*)a.gy, (T*)a.phi, a.ctrl);
             else if constexpr (sizeof(T) == 4)

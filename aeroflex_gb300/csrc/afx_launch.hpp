@@ -54,6 +54,11 @@ struct Prof {
     }
 };
 
+// Four lanes per cell in k_prep and k_limiter?  Below 40,000 cells.  16k cells,
+// FP64: k_prep 19.7 -> 13.8 us, k_limiter 9.1 -> 6.5; 17k, FP32: 7.2 -> 4.8, 5.8 ->
+// 3.8; 74k, FP64: 44.2 against 47.7 and 16.7 against 17.3 with four.
+inline bool four_lanes(int n_cells) { return n_cells < 40000; }
+
 // Everything a launch needs.  Pointers to typed arrays are passed as void*
 // and cast in the precision's translation unit (T = double or float).
 struct StepArgs {
@@ -68,7 +73,7 @@ struct StepArgs {
     const void* fd0 = nullptr;    // T2 [F]
     const void* fd1 = nullptr;    // T2 [F]
     const void* ft = nullptr;     // T4 [F]
-    const void* dsl = nullptr;    // T2 [4N] (FP32): face centre - centroid per cell slot, slot-major
+    const void* dsl = nullptr;    // T2 [4N] (FP32, unless four_lanes): face centre - centroid per cell slot, slot-major
     const void* btype = nullptr;  // int [B]
     const void* bq = nullptr;     // T4 [B] ghost (boundary) states
     // physics / scheme
